@@ -34,6 +34,24 @@ __host__ __device__ inline unsigned grid_for(long long n, int block = kBlock) {
     return (unsigned)(g > 0 ? g : 1);
 }
 
+// Threads per block of a launch with n independent threads (one cell or
+// block row each) of type T, at most cap (a tuned launch; 0: none).  A SM
+// sub-partition issues one FP64 warp instruction per 64 clocks (2 lanes per
+// clock and SM), so the time of a small level is the warps of the busiest
+// sub-partition times their instructions: with 256 threads per block a level
+// of 1000 cells ran on 4 of the 152 SMs, two warps to a sub-partition.  One
+// warp per block while every warp can have a sub-partition to itself; two
+// warps per block up to four warps per sub-partition, where whole blocks of
+// 256 would leave SMs with one block more than others.
+template <typename T>
+__host__ inline int spread_block(long long n, int cap) {
+    constexpr long long kParts = 4 * 152;  // SM sub-partitions
+    const int most = cap > 0 ? cap : (sizeof(T) == 8 ? 64 : 256);
+    const long long warps = (n + 31) / 32;
+    const int want = warps <= kParts ? 32 : warps <= 4 * kParts ? 64 : most;
+    return want < most ? want : most;
+}
+
 // Block-wide sum of a double (blockDim.x multiple of 32, <= 1024); result
 // valid in thread 0.
 __device__ inline double block_sum(double v) {

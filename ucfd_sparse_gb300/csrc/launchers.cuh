@@ -18,11 +18,12 @@ void adj_upper(const ::ucfd::AdjArgs &a, int nfv, int ndims, T gamma, T pmin, co
                T *gfspr, cudaStream_t s) {
     const int n = a.t1 - a.t0;
     if (n <= 0) return;
+    const int block = spread_block<T>(n, 0);
     if (nfv == 5 && ndims == 3)
-        adj_upper_kernel<T, 5, 5, 3><<<grid_for(n), kBlock, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag, dub,
+        adj_upper_kernel<T, 5, 5, 3><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag, dub,
                                                                      dq, gdq, qbar, dbar, gfspr);
     else if (nfv == 4 && ndims == 2)
-        adj_upper_kernel<T, 4, 4, 2><<<grid_for(n), kBlock, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag, dub,
+        adj_upper_kernel<T, 4, 4, 2><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag, dub,
                                                                      dq, gdq, qbar, dbar, gfspr);
     else
         ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "adjoint built for nfvars/ndims 5/3 and 4/2 only");
@@ -34,11 +35,12 @@ void adj_lower(const ::ucfd::AdjArgs &a, int nfv, int ndims, T gamma, T pmin, T 
                const T *dbar, T *grhs, T *gdt, T *gfspr, cudaStream_t s) {
     const int n = a.t1 - a.t0;
     if (n <= 0) return;
+    const int block = spread_block<T>(n, 0);
     if (nfv == 5 && ndims == 3)
-        adj_lower_kernel<T, 5, 5, 3><<<grid_for(n), kBlock, 0, s>>>(a, gamma, pmin, factor, fnv, vec, fspr, dt, upts,
+        adj_lower_kernel<T, 5, 5, 3><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, factor, fnv, vec, fspr, dt, upts,
                                                                      diag, dub, qbar, wbuf, dbar, grhs, gdt, gfspr);
     else if (nfv == 4 && ndims == 2)
-        adj_lower_kernel<T, 4, 4, 2><<<grid_for(n), kBlock, 0, s>>>(a, gamma, pmin, factor, fnv, vec, fspr, dt, upts,
+        adj_lower_kernel<T, 4, 4, 2><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, factor, fnv, vec, fspr, dt, upts,
                                                                      diag, dub, qbar, wbuf, dbar, grhs, gdt, gfspr);
     else
         ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "adjoint built for nfvars/ndims 5/3 and 4/2 only");
@@ -118,7 +120,8 @@ static void sweep_both_go(const ::ucfd::ScalarSweepArgs<T> &a, int block, cudaSt
 template <typename T>
 void scalar_sweep(const ::ucfd::ScalarSweepArgs<T> &a, int nv, int nfv, int ndims, int rans,
                   int block, cudaStream_t s) {
-    if (block <= 0) block = kBlock;
+    if (a.facelist) block = block > 0 ? block : kBlock;
+    else block = spread_block<T>(a.pair ? 2ll * (a.t1 - a.t0) : a.t1 - a.t0, block);
 #define UCFD_SW(NV, NFV, ND)                                                   \
     if (nv == NV && nfv == NFV && ndims == ND) {                               \
         if (rans == 2) {                                                       \
@@ -306,7 +309,8 @@ void fs_blusgs_prepare(int B, long long N, int P, long long nF, const int *nei, 
     if (N <= 0) return;
     const unsigned gt = (unsigned)((nF + 31) / 32);
     UCFD_BSW(B, (jmat_face_major_kernel<BB><<<gt, 256, 0, s>>>(nF, jmat, jt)));
-    UCFD_BSW(B, (fs_blusgs_prepare_kernel<S, BB><<<grid_for(N, 128), 128, 0, s>>>(
+    const int block = spread_block<double>(N, 128);
+    UCFD_BSW(B, (fs_blusgs_prepare_kernel<S, BB><<<grid_for(N, block), block, 0, s>>>(
                     N, P, nei, slot, side, fa, rv, jt, dd, D, LU64, LU_s, J_s, J64)));
 }
 
@@ -384,7 +388,7 @@ void fs_blusgs_sweep(int B, int t0, int t1, long long N, int P, int var0, const 
                      int variant, int *err, long long max_spin, const ::ucfd::SweepSplit<S> &sp,
                      cudaStream_t s) {
     if (t1 <= t0) return;
-    if (block <= 0) block = kBlock;
+    block = spread_block<S>(t1 - t0, block);
     // threads start at the tile boundary below t0 (see the kernel)
     const unsigned g = grid_for(t1 - (t0 & ~31), block);
     // variant 0: faces unrolled to the ELL width (6 or 4) when it matches;
@@ -487,7 +491,7 @@ template <typename Tv, typename Ta>
 void bsr_spmv(int B, int bn, int P, const int *col, const Tv *val, double alpha, const double *x,
               double beta, double *y, int block, cudaStream_t s) {
     if (bn <= 0) return;
-    if (block <= 0) block = kBlock;
+    block = spread_block<Ta>(bn, block);
     const unsigned g = grid_for(bn, block);
     // unrolled rows for the 5x5 systems (tets: diag + 4 faces; hexes: + 6)
     if (B == 5 && P <= 5) {
@@ -505,7 +509,8 @@ template <typename Tl>
 void pc_prepare(int B, int bn, const int *perm, const long long *dslot, const double *values,
                 double *LU64, Tl *LU_l, int factor, cudaStream_t s) {
     if (bn <= 0) return;
-    UCFD_KSW(B, (pc_prepare_kernel<Tl, BB><<<grid_for(bn, 128), 128, 0, s>>>(bn, perm, dslot, values, LU64,
+    const int block = spread_block<double>(bn, 128);
+    UCFD_KSW(B, (pc_prepare_kernel<Tl, BB><<<grid_for(bn, block), block, 0, s>>>(bn, perm, dslot, values, LU64,
                                                                              LU_l, factor)));
 }
 
@@ -553,7 +558,7 @@ template <typename T, bool LOWER>
 static void pc_step(int B, int t0, int t1, int bn, int P, const int *col, const T *val, const T *LU, T *b,
                     int block, int mode, cudaStream_t s) {
     if (t1 <= t0) return;
-    if (block <= 0) block = kBlock;
+    block = spread_block<T>(t1 - t0, block);
     const unsigned g = grid_for(t1 - t0, block);
     if (mode == PC_BILU) pc_step_go<T, PC_BILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, b);
     else if (mode == PC_ILU) pc_step_go<T, PC_ILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, b);
@@ -576,13 +581,14 @@ void pc_upper(int B, int t0, int t1, int bn, int PU, const int *Ucol, const T *U
 void ilu_factor(int B, int scalar, int t0, int t1, const int *rows, const int *rowptr, const int *colidx,
                 const int *diagslots, double *vals, cudaStream_t s) {
     if (t1 <= t0) return;
-    const unsigned g = grid_for(t1 - t0, 128);
+    const int block = spread_block<double>(t1 - t0, 0);
+    const unsigned g = grid_for(t1 - t0, block);
     if (scalar) {
         if (B != 1) ::ucfd::fail(UCFD_ERR_ARGUMENT, "scalar ILU needs block size 1 (got %d)", B);
-        ilu_factor_kernel<1, true><<<g, 128, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
+        ilu_factor_kernel<1, true><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
         return;
     }
-    UCFD_KSW(B, (ilu_factor_kernel<BB, false><<<g, 128, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals)));
+    UCFD_KSW(B, (ilu_factor_kernel<BB, false><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals)));
 }
 
 template <typename Ts, typename Td>
