@@ -319,36 +319,61 @@ __global__ void scatter_rows_kernel(int bn, int B, const int *perm, const Ts *sr
 constexpr int kMaxK = 32;  // restart length + 1 <= kMaxK
 
 // Grid of the reduction kernels: capped so the per-block partial buffers
-// stay small (8 blocks x 152 SMs).
+// stay small (8 blocks x 152 SMs), and below that one block per SM before a
+// block gets fewer than 8 values per thread: a block's own reduction costs
+// as many FP64 instructions as several values, and the last block sums one
+// partial per block.
 constexpr int kRedBlocks = 1216;
 __host__ __device__ inline int gm_grid(long long n) {
     const long long g = (n + kBlock - 1) / kBlock;
-    return (int)(g < kRedBlocks ? (g > 0 ? g : 1) : kRedBlocks);
+    if (g <= 152) return (int)(g > 0 ? g : 1);
+    const long long few = (n + 8 * kBlock - 1) / (8 * kBlock);
+    return (int)(few < 152 ? 152 : few < kRedBlocks ? few : kRedBlocks);
 }
 
-// Per-block partial dots h[k] = sum_i V[k][i] * w[i], k < K.
+// Grid of the vector updates without a reduction (grid-stride).
+__host__ inline unsigned vec_grid(long long n) {
+    const unsigned g = grid_for(n);
+    return g < kRedBlocks ? g : kRedBlocks;
+}
+
+// Block sums of KM per-thread accumulators (only the first KK meaningful;
+// 256 threads), sum k to part[k].  Eight accumulators at a time go through
+// shared memory: warp w adds the 256 values of accumulator w, eight per
+// lane, then one shuffle tree.  That is 13 FP64 warp additions per
+// accumulator and block against 40 with one shuffle tree per warp and
+// accumulator, which on GB300's FP64 pipe (one warp instruction per 64
+// clocks and SM sub-partition) outweighed the sums themselves in short
+// vectors: five sums of 414,000 values 24.7 -> 10.8 us
+// (with the smaller grid of gm_grid).
+template <int KM>
+__device__ __forceinline__ void block_sum_many(const double *acc, int KK, double *part) {
+    constexpr int CH = KM < 8 ? KM : 8;
+    __shared__ double sm[CH][kBlock];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int k0 = 0; k0 < KM; k0 += CH) {
+        if (k0 > 0) __syncthreads();  // the previous sums are read
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+            if (k0 + c < KM) sm[c][threadIdx.x] = acc[k0 + c];
+        __syncthreads();
+        if (wid < CH && k0 + wid < KK) {
+            double v = sm[wid][lane];
+#pragma unroll
+            for (int q = 1; q < kBlock / 32; ++q) v += sm[wid][q * 32 + lane];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) part[k0 + wid] = v;
+        }
+    }
+}
+
 // Block partials of KM accumulators (only the first KK meaningful) into
 // part[block][k].
 template <int KM>
 __device__ __forceinline__ void gm_block_partials(const double *acc, int KK, double *part) {
-    __shared__ double sm[KM][9];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < KM; ++k) {
-        if (k < KK) {
-            double v = acc[k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) sm[k][wid] = v;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < KK) {
-        double s = 0.0;
-        const int nw = blockDim.x >> 5;
-        for (int q = 0; q < nw; ++q) s += sm[threadIdx.x][q];
-        part[(long long)blockIdx.x * kMaxK + threadIdx.x] = s;
-    }
+    block_sum_many<KM>(acc, KK, part + (long long)blockIdx.x * kMaxK);
 }
 
 // Basis vectors whose entries a thread of the orthogonalisation kernels
@@ -652,9 +677,9 @@ __global__ void __launch_bounds__(256) bc_dot_kernel(long long n, const double *
 
 // rho_0 = (r~, r_0), rhoprev = alpha = omega = 1 (bicgstab.c:52-56); a
 // rho breakdown (|rho| < 1e-30, bicgstab.c:59-62) ends the solve.
-__global__ void bc_start_kernel(int nb, const double *part, BcState *st, int maxiter) {
-    double rho = 0.0;
-    for (int b = 0; b < nb; ++b) rho += part[b];
+__global__ void __launch_bounds__(256) bc_start_kernel(int nb, const double *part, BcState *st, int maxiter) {
+    const double rho = block_sum_partials(part, nb, 1);
+    if (threadIdx.x != 0) return;
     st->rho = rho;
     st->rhoprev = 1.0;
     st->alpha = 1.0;
@@ -697,10 +722,10 @@ __global__ void __launch_bounds__(256) bc_direction_kernel(long long n, const Bc
 }
 
 // pi = (r~, v); alpha = rho / pi, or a pi breakdown (bicgstab.c:81-86).
-__global__ void bc_alpha_kernel(int nb, const double *part, BcState *st) {
-    if (st->stop) return;
-    double pi = 0.0;
-    for (int b = 0; b < nb; ++b) pi += part[b];
+__global__ void __launch_bounds__(256) bc_alpha_kernel(int nb, const double *part, BcState *st) {
+    if (st->stop) return;  // the same for every thread of the block
+    const double pi = block_sum_partials(part, nb, 1);
+    if (threadIdx.x != 0) return;
     if (fabs(pi) < 1e-30) {
         st->stat = 4;
         st->stop = 1;
@@ -737,35 +762,27 @@ __global__ void __launch_bounds__(256) bc_fused5_kernel(long long n, const doubl
         d += tk * tk;
         e += sk * sk;
     }
-    a = block_sum(a);
-    b = block_sum(b);
-    c = block_sum(c);
-    d = block_sum(d);
-    e = block_sum(e);
-    if (threadIdx.x == 0) {
-        double *q = part + 5ll * blockIdx.x;
-        q[0] = a;
-        q[1] = b;
-        q[2] = c;
-        q[3] = d;
-        q[4] = e;
-    }
+    const double acc[5] = {a, b, c, d, e};
+    block_sum_many<5>(acc, 5, part + 5ll * blockIdx.x);
 }
 
 // omega = (t,s)/(t,t), rho_new = phi - omega (r~,t) and the residual
 // estimate sqrt|ss - 2 omega ts + omega^2 tt| (bicgstab.c:101-118);
 // conv when it is below tol.
-__global__ void bc_omega_kernel(int nb, const double *part, BcState *st, double tol, double *hist) {
-    if (st->stop) return;
-    double phi = 0.0, rtt = 0.0, ts = 0.0, tt = 0.0, ss = 0.0;
-    for (int b = 0; b < nb; ++b) {
-        const double *q = part + 5ll * b;
-        phi += q[0];
-        rtt += q[1];
-        ts += q[2];
-        tt += q[3];
-        ss += q[4];
-    }
+// The partials are summed by a whole block (one thread adding 5 x 1216 of
+// them in a chain took 335 us; now 5.1 us).
+__global__ void __launch_bounds__(256) bc_omega_kernel(int nb, const double *part, BcState *st, double tol,
+                                                       double *hist) {
+    if (st->stop) return;  // the same for every thread of the block
+    __shared__ double sums[5];
+    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < nb; b += blockDim.x)
+#pragma unroll
+        for (int j = 0; j < 5; ++j) acc[j] += part[5ll * b + j];
+    block_sum_many<5>(acc, 5, sums);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double phi = sums[0], rtt = sums[1], ts = sums[2], tt = sums[3], ss = sums[4];
     // (t, t) == 0 means s == 0 (t = A inv(M) s): x + alpha pt already solves
     // the system.  The reference divides regardless (0/0 = NaN, after which
     // it never converges); omega = 0 gives r = s = 0 and a zero estimate.

@@ -668,7 +668,7 @@ void gm_cycle_begin(int nblocks, const double *part, void *st, double *y, double
 }
 
 void gm_scale(long long n, const void *st, const double *src, double *dst, cudaStream_t s) {
-    gm_scale_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, (const GmState *)st, src, dst);
+    gm_scale_kernel<<<vec_grid(n), kBlock, 0, s>>>(n, (const GmState *)st, src, dst);
 }
 
 void gm_givens(int j, int ld, int nblocks, const double *part_norm, double *H, const double *h2, double *cs,
@@ -683,7 +683,7 @@ void gm_backsub(int ld, const double *H, double *y, const void *st, cudaStream_t
 
 void gm_solution(long long n, const double *V, long long ldv, const double *y, const void *st, double *x,
                  cudaStream_t s) {
-    gm_solution_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, V, ldv, y, (const GmState *)st, x);
+    gm_solution_kernel<<<vec_grid(n), kBlock, 0, s>>>(n, V, ldv, y, (const GmState *)st, x);
 }
 
 size_t gm_state_bytes() { return sizeof(GmState); }
@@ -794,29 +794,29 @@ void bc_dot(long long n, const double *x, const double *y, double *part, const v
     bc_dot_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, x, y, part, (const BcState *)st);
 }
 void bc_start(int nb, const double *part, void *st, int maxiter, cudaStream_t s) {
-    bc_start_kernel<<<1, 1, 0, s>>>(nb, part, (BcState *)st, maxiter);
+    bc_start_kernel<<<1, kBlock, 0, s>>>(nb, part, (BcState *)st, maxiter);
 }
 void bc_direction(long long n, const void *st, const double *r, const double *v, double *p, double *pt,
                   cudaStream_t s) {
-    bc_direction_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, (const BcState *)st, r, v, p, pt);
+    bc_direction_kernel<<<vec_grid(n), kBlock, 0, s>>>(n, (const BcState *)st, r, v, p, pt);
 }
 void bc_alpha(int nb, const double *part, void *st, cudaStream_t s) {
-    bc_alpha_kernel<<<1, 1, 0, s>>>(nb, part, (BcState *)st);
+    bc_alpha_kernel<<<1, kBlock, 0, s>>>(nb, part, (BcState *)st);
 }
 void bc_s(long long n, const void *st, const double *r, const double *v, double *sv, double *shat,
           cudaStream_t s) {
-    bc_s_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, (const BcState *)st, r, v, sv, shat);
+    bc_s_kernel<<<vec_grid(n), kBlock, 0, s>>>(n, (const BcState *)st, r, v, sv, shat);
 }
 void bc_fused5(long long n, const double *rt, const double *sv, const double *t, double *part, const void *st,
                cudaStream_t s) {
     bc_fused5_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, rt, sv, t, part, (const BcState *)st);
 }
 void bc_omega(int nb, const double *part, void *st, double tol, double *hist, cudaStream_t s) {
-    bc_omega_kernel<<<1, 1, 0, s>>>(nb, part, (BcState *)st, tol, hist);
+    bc_omega_kernel<<<1, kBlock, 0, s>>>(nb, part, (BcState *)st, tol, hist);
 }
 void bc_update(long long n, const void *st, const double *pt, const double *shat, const double *sv,
                const double *t, double *x, double *r, cudaStream_t s) {
-    bc_update_kernel<<<gm_blocks(n), kBlock, 0, s>>>(n, (const BcState *)st, pt, shat, sv, t, x, r);
+    bc_update_kernel<<<vec_grid(n), kBlock, 0, s>>>(n, (const BcState *)st, pt, shat, sv, t, x, r);
 }
 void bc_advance(void *st, int maxiter, cudaStream_t s) {
     bc_advance_kernel<<<1, 1, 0, s>>>((BcState *)st, maxiter);
