@@ -91,6 +91,7 @@ struct _FlowSys {
     DevBuf<double> D, dd, LU64, tD, tLU64, J64, rhs64, x64;  // FP64 block arrays
     DevBuf<double> jt;  // Prepare scratch: face Jacobians, one record per face
     DevBuf<int> d_sweep_err;  // set by a bulk-copy block sweep whose copy wait gave up
+    bool bulk_swept = false;  // a bulk-copy variant ran since d_sweep_err was last read
     bool du64_valid = false;
     bool c_valid[2] = {false, false};  // crhs of the NS / turbulence rows matches rhs and the factors
     bool x_zero = false;  // the correction du is all zeros (Reset, no sweep since)
@@ -438,8 +439,11 @@ void blusgs_alloc(FlowSys s) {
 
 // Bulk-copy sweeps report a copy wait that gave up through d_sweep_err;
 // read (and clear) it at the points where the host synchronises anyway.
+// Only those variants (2 and 3) wait for a copy; after the others there is
+// nothing to read, which saves a copy and a second synchronisation per call.
 void check_sweep_err(FlowSys s) {
-    if (!s->d_sweep_err.p) return;
+    if (!s->d_sweep_err.p || !s->bulk_swept) return;
+    s->bulk_swept = false;
     int err = 0;
     UCFD_CUDA(cudaMemcpyAsync(&err, s->d_sweep_err.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream()));
     UCFD_CUDA(cudaStreamSynchronize(s->stream()));
@@ -493,6 +497,7 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
         sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0])
                       ? 0 : 1;
     }
+    if (s->variant == 2 || s->variant == 3) s->bulk_swept = true;
     for (int q = 0; q < L; ++q) {
         const int l = upper ? L - 1 - q : q;
         KCALL(EX, fs_blusgs_sweep<S>, B, s->sch.lev_off[l], s->sch.lev_off[l + 1], s->N, s->P, var0,
