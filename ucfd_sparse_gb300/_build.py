@@ -71,7 +71,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     def compile_one(unit):
         src, extra = unit
         obj = os.path.join(BUILD, os.path.splitext(src)[0] + ".o")
-        cmd = [cc, *ARCH, *COMMON, *extra, "-c", os.path.join(CSRC, src), "-o", obj]
+        # the kernel units: optimised in parallel parts (halves the longest unit's build time)
+        split = ["--split-compile=0"] if src.endswith(".cu") else []
+        cmd = [cc, *ARCH, *COMMON, *split, *extra, "-c", os.path.join(CSRC, src), "-o", obj]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed for {src}:\n{' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
