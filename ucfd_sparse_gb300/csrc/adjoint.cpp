@@ -43,10 +43,13 @@ void step(int neles, int nface, int nvars, int nfvars, int ndims, const int *nei
         a.nbsrc = upper ? dq : dub;
         a.own_in = upper ? dub : rhs;
         a.own_out = upper ? dq : dub;
+        bool launched = false;
         for (int q = 0; q < ncolors; ++q) {
             const int c = upper ? ncolors - 1 - q : q;
             a.t0 = c == 0 ? 0 : ranges[c - 1];
             a.t1 = ranges[c];
+            a.chained = launched;
+            launched = launched || a.t1 > a.t0;
             if constexpr (EX) kexact::scalar_sweep<T>(a, nvars, nfvars, ndims, 0, 0, s);
             else kfast::scalar_sweep<T>(a, nvars, nfvars, ndims, 0, 0, s);
         }

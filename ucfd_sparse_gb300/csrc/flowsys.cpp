@@ -98,6 +98,7 @@ struct _FlowSys {
     SplitState split[2];           // NS / turbulence rows of the fast block sweeps
     unsigned jver[2] = {1, 1};     // Prepare count of the NS / turbulence blocks
     bool has_self = false;         // some CSR row lists itself
+    std::vector<int> act[2];       // per level: most faces of a cell towards earlier / later levels
     bool lam2_ok = false;          // Work::lam2 packs the current NS and RANS spectral radii (FP32)
     DevBuf<double> part, red, resid;
     PinnedBuf<double> h_red;
@@ -172,6 +173,18 @@ void build_topology(FlowSys s) {
         sort_levels_by(s->sch, bfs);
     }
     const Schedule &sch = s->sch;
+    for (std::vector<int> &v : s->act) v.assign(sch.nlev, 0);
+    for (int l = 0; l < sch.nlev; ++l)
+        for (int k = sch.lev_off[l]; k < sch.lev_off[l + 1]; ++k) {
+            int n0 = 0, n1 = 0;
+            for (int q = rp[sch.perm[k]]; q < rp[sch.perm[k] + 1]; ++q) {
+                const int nb = sch.iperm[ci[q]];
+                n0 += nb < sch.lev_off[l];
+                n1 += nb >= sch.lev_off[l + 1];
+            }
+            s->act[0][l] = std::max(s->act[0][l], n0);
+            s->act[1][l] = std::max(s->act[1][l], n1);
+        }
     int P = 0;
     for (int i = 0; i < n; ++i) P = std::max(P, rp[i + 1] - rp[i]);
     P = std::max(P, 1);
@@ -380,12 +393,16 @@ void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent =
               s->d_bar.p, s->d_err.p, kBarrierMaxSpin, s->stream());
         return;
     }
+    bool launched = false;
     for (int q = 0; q < L; ++q) {
         const int l = upper ? L - 1 - q : q;
         a.t0 = s->sch.lev_off[l];
         a.t1 = s->sch.lev_off[l + 1];
         a.lo = a.t0;
         a.hi = a.t1;
+        a.max_active = std::max(s->act[upper ? 1 : 0][l], 1);
+        a.chained = launched;
+        launched = launched || a.t1 > a.t0;
         KCALL(EX, scalar_sweep<S>, a, s->nvars, s->nfvars, s->ndims, sys, s->block, s->stream());
     }
 }

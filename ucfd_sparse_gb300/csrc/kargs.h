@@ -61,6 +61,9 @@ struct ScalarSweepArgs {
     int upper;
     int regcap;            // 0, or 3 / 4: the kernel built for that many blocks of 256 threads per SM
                            // (at most 80 / 64 registers)
+    int max_active;        // most faces any cell of the range has towards this sweep's earlier levels
+                           // (0: not known, up to nface)
+    int chained;           // 1: the previous launch on the stream is the previous level of the same sweep
     int pair;              // 1: two threads per cell (faces 0-2 / 3-5; ELL width <= 6, per-level launches)
     // one thread per active face (per-level launches): the faces of this
     // sweep direction whose neighbour lies in an earlier level, cell by cell

@@ -42,7 +42,10 @@ __host__ __device__ inline unsigned grid_for(long long n, int block = kBlock) {
 // of 1000 cells ran on 4 of the 152 SMs, two warps to a sub-partition.  One
 // warp per block while every warp can have a sub-partition to itself; two
 // warps per block up to four warps per sub-partition, where whole blocks of
-// 256 would leave SMs with one block more than others.
+// 256 would leave SMs with one block more than others.  Measured against
+// blocks of 256: array LU-SGS step of 32^3 cells (two colours of 16384) 250 ->
+// 198 us, natural-order step of 41x36x33 cells (108 levels of at most 1100)
+// 6.44 -> 4.04 ms, both FP64.
 template <typename T>
 __host__ inline int spread_block(long long n, int cap) {
     constexpr long long kParts = 4 * 152;  // SM sub-partitions

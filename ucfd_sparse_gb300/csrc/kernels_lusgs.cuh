@@ -22,6 +22,27 @@ namespace UCFD_KNS {
 __device__ __forceinline__ float div_sweep(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double div_sweep(double a, double b) { return a / b; }
 
+// x * y rounded on its own (never fused into a following add), so that
+// every sweep kernel forms the same per-face term whatever the compiler
+// contracts; with contraction off this is the plain product.
+__device__ __forceinline__ float mul_rn(float x, float y) { return __fmul_rn(x, y); }
+__device__ __forceinline__ double mul_rn(double x, double y) { return __dmul_rn(x, y); }
+
+// a b + c d, in the fast build with one fused multiply-add (the same one in
+// every sweep kernel).
+template <typename T>
+__device__ __forceinline__ T sum_prod(T a, T b, T c, T d) {
+    if constexpr (kFold) return fma(a, b, mul_rn(c, d));
+    else return a * b + c * d;
+}
+
+// acc + a b, in the fast build one fused multiply-add.
+template <typename T>
+__device__ __forceinline__ T add_prod(T acc, T a, T b) {
+    if constexpr (kFold) return fma(a, b, acc);
+    else return acc + a * b;
+}
+
 // ns_flux_container: flux.c:29-67.  The pressure floor rewrites the energy
 // of the local copy u (flux.c:51-56), exactly as the reference does.  In
 // FP32 the two divisions by rho are products with one reciprocal.
@@ -32,8 +53,8 @@ __device__ __forceinline__ void ns_flux(T gamma, T pmin, T *u, const T *nf, T *f
     T temp = T(0), contrav = T(0);
 #pragma unroll
     for (int i = 0; i < NDIMS; ++i) {
-        contrav += u[i + 1] * nf[i];
-        temp += u[i + 1] * u[i + 1];
+        contrav = add_prod(contrav, u[i + 1], nf[i]);
+        temp = add_prod(temp, u[i + 1], u[i + 1]);
     }
     T ke;  // 0.5 * temp / rho
     if constexpr (sizeof(T) == 4) {
@@ -44,17 +65,17 @@ __device__ __forceinline__ void ns_flux(T gamma, T pmin, T *u, const T *nf, T *f
         contrav /= rho;
         ke = T(0.5) * temp / rho;
     }
-    T p = (gamma - T(1)) * (et - ke);
+    T p = mul_rn(gamma - T(1), et - ke);
     if (p < pmin) {
         p = pmin;
         et = p / (gamma - T(1)) + ke;
         u[NFV - 1] = et;
     }
     T ht = et + p;
-    f[0] = rho * contrav;
+    f[0] = mul_rn(rho, contrav);
 #pragma unroll
-    for (int i = 0; i < NDIMS; ++i) f[i + 1] = u[i + 1] * contrav + nf[i] * p;
-    f[NFV - 1] = ht * contrav;
+    for (int i = 0; i < NDIMS; ++i) f[i + 1] = sum_prod(u[i + 1], contrav, nf[i], p);
+    f[NFV - 1] = mul_rn(ht, contrav);
 }
 
 // rans_flux_container: flux.c:77-90
@@ -63,10 +84,10 @@ __device__ __forceinline__ void rans_flux(const T *u, const T *nf, T *f) {
     T rho = u[0];
     T contrav = T(0);
 #pragma unroll
-    for (int i = 0; i < NDIMS; ++i) contrav += u[i + 1] * nf[i];
+    for (int i = 0; i < NDIMS; ++i) contrav = add_prod(contrav, u[i + 1], nf[i]);
     contrav = div_sweep(contrav, rho);
 #pragma unroll
-    for (int i = 0; i < NT; ++i) f[i] = u[NFV + i] * contrav;
+    for (int i = 0; i < NT; ++i) f[i] = mul_rn(u[NFV + i], contrav);
 }
 
 // F(u + dn; n) - F(u; n) of ns_flux in difference form, for FP32: the
@@ -209,12 +230,6 @@ __global__ void __launch_bounds__(256, MINB) scalar_sweep_persistent_kernel(Scal
         if (q + 1 < nlev && !grid_barrier_bounded(bar, bar + 1, err, max_spin)) return;
     }
 }
-
-// x * y rounded on its own (never fused into a following add), so that
-// every sweep kernel forms the same per-face term whatever the compiler
-// contracts; with contraction off this is the plain product.
-__device__ __forceinline__ float mul_rn(float x, float y) { return __fmul_rn(x, y); }
-__device__ __forceinline__ double mul_rn(double x, double y) { return __dmul_rn(x, y); }
 
 // Active faces among the NB face slots f0 .. f0+NB-1 of a cell (neighbours
 // nb[q], -1 for none): bit q is set when the neighbour of slot q belongs to
@@ -523,6 +538,136 @@ __device__ __forceinline__ void scalar_sweep_cell_both(const ScalarSweepArgs<T> 
     }
 #pragma unroll
     for (int k = 0; k < NV; ++k) a.own_out[k * ld + i] = sweep_result(a.upper != 0, own[k], df[k], dg[k]);
+}
+
+// ---- FP64 sweep of a small level: two lanes per active face ------------------
+// A SM sub-partition issues one FP64 warp instruction per 64 clocks whatever
+// the number of its active lanes, so a level with fewer warps than
+// sub-partitions costs the FP64 instructions of one thread: about 480 (15 us)
+// with one thread per cell.  Here GF pairs of lanes share a cell, one pair
+// per active face.  The two dot products of a flux (m.n and m.m), its two
+// divisions by rho and its components are split between the lanes of a pair;
+// the terms meet in shared memory, where lane v of the cell adds variable v
+// in face order.  About 95 instructions per warp, a third of them (the flux
+// of the neighbour's state, which the sweep does not change) before
+// griddepcontrol.wait.  Every operation and its operands are those of
+// scalar_sweep_cell (a sum's leading 0 + x is dropped, which can only change
+// the sign of a zero), so the values are the same.
+template <int NFV, int NDIMS>
+__device__ __forceinline__ void ns_flux_lane(double gamma, double pmin, const double *u, const double *n, int h,
+                                             double *fx) {
+    double dot = mul_rn(u[1], h ? u[1] : n[0]);
+#pragma unroll
+    for (int d = 1; d < NDIMS; ++d) dot = add_prod(dot, u[d + 1], h ? u[d + 1] : n[d]);
+    const double q = mul_rn(h ? 0.5 : 1.0, dot) / u[0];  // lane 0: m.n / rho; lane 1: 0.5 m.m / rho
+    const double o = __shfl_xor_sync(0xffffffffu, q, 1);
+    const double c = h ? o : q, ke = h ? q : o;
+    double et = u[NFV - 1];
+    double p = mul_rn(gamma - 1.0, et - ke);
+    if (p < pmin) {
+        p = pmin;
+        et = p / (gamma - 1.0) + ke;
+    }
+    fx[0] = mul_rn(h ? et + p : u[0], c);
+    fx[1] = sum_prod(h ? u[NDIMS] : u[1], c, h ? n[NDIMS - 1] : n[0], p);
+    fx[2] = NDIMS == 3 ? sum_prod(u[2], c, n[1], p) : 0.0;  // lane 0 only
+}
+
+template <int NV, int NFV, int NDIMS, bool RANS, int GF>
+__device__ __forceinline__ void scalar_sweep_lanes(const ScalarSweepArgs<double> &a, double *sm) {
+    constexpr int NV0 = RANS ? NFV : 0;
+    constexpr int DNV = RANS ? NV - NFV : NFV;
+    constexpr int G = 2 * GF;  // lanes per cell
+    constexpr int NB = 8;      // face slots of a row
+    const long long ld = a.ld;
+    const int g = threadIdx.x % G, k = g >> 1, h = g & 1;
+    const int t = a.t0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) / G);
+    const bool valid = t < a.t1;
+    const int i = valid ? (a.cells ? __ldg(a.cells + t) : t) : 0;
+    const int ci = a.lcolor ? __ldg(a.lcolor + i) : 0;
+    double *terms = sm + (threadIdx.x / G) * (GF * DNV);  // [GF][DNV] of this cell
+
+    // everything the previous level does not write
+    int nb[NB];
+#pragma unroll
+    for (int p = 0; p < NB; ++p) nb[p] = valid && p < a.nface ? __ldg(a.nei + p * ld + i) : -1;
+    unsigned m = valid && !no_active_face(a, a.lo, a.hi) ? active_faces<double, NB>(a, a.lo, a.hi, ci, nb) : 0u;
+    const int count = __popc(m);
+    for (int q = 0; q < k; ++q) m &= m - 1u;
+    const bool on = m != 0u;
+    const int f = on ? __ffs(m) - 1 : 0;
+    int j = i;
+#pragma unroll
+    for (int p = 0; p < NB; ++p) j = on && f == p ? nb[p] : j;
+    double own = 0.0, dg = 1.0;
+    if (valid && g < DNV) {
+        own = a.own_in[(g + NV0) * ld + i];
+        dg = a.diag[(g + NV0) * a.diag_vs + i];
+    }
+    double u[NV], n[NDIMS];
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+        u[v] = flux_reads<double, NV, NFV, NDIMS, RANS>(v) ? __ldg(a.u + v * ld + j) : 0.0;
+#pragma unroll
+    for (int d = 0; d < NDIMS; ++d) n[d] = __ldg(a.nrm + (f * NDIMS + d) * ld + i);
+    const double fv = __ldg(a.fa + f * ld + i);
+    const double fvk = a.rv ? fv * __ldg(a.rv + i) : fv;
+    const double klk = a.kappa * __ldg(a.lam + f * ld + i);
+    if constexpr (RANS) {
+        // lane h of the pair: turbulence variable h
+        double c = mul_rn(u[1], n[0]);
+#pragma unroll
+        for (int d = 1; d < NDIMS; ++d) c = add_prod(c, u[d + 1], n[d]);
+        c /= u[0];
+        const double ut = h && DNV > 1 ? u[NV - 1] : u[NFV];
+        const double f0 = mul_rn(ut, c);
+        if (a.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (on && h < DNV) {
+            const double dn = __ldcg(a.nbsrc + (h + NV0) * ld + j);
+            const double dfl = mul_rn(dn + ut, c) - f0;
+            terms[k * DNV + h] = mul_rn(dfl - klk * dn, fvk);
+        }
+    } else {
+        double f0[3], f1[3], dn[NFV], w[NFV];
+        ns_flux_lane<NFV, NDIMS>(a.gamma, a.pmin, u, n, h, f0);
+        if (a.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+        for (int v = 0; v < NFV; ++v) dn[v] = on ? __ldcg(a.nbsrc + v * ld + j) : 0.0;
+#pragma unroll
+        for (int v = 0; v < NFV; ++v) w[v] = dn[v] + u[v];
+        ns_flux_lane<NFV, NDIMS>(a.gamma, a.pmin, w, n, h, f1);
+        if (on) {
+            double *o = terms + k * DNV;
+            const double e0 = h ? dn[NFV - 1] : dn[0], e1 = h ? dn[NDIMS] : dn[1];
+            o[h ? NFV - 1 : 0] = mul_rn((f1[0] - f0[0]) - klk * e0, fvk);
+            o[h ? NDIMS : 1] = mul_rn((f1[1] - f0[1]) - klk * e1, fvk);
+            if (NDIMS == 3 && !h) o[2] = mul_rn((f1[2] - f0[2]) - klk * dn[2], fvk);
+        }
+    }
+    __syncwarp();
+    if (!valid || g >= DNV) return;
+    double df = 0.0;
+    if (count > 0) {
+        df = terms[g];
+        for (int q = 1; q < count; ++q) df += terms[q * DNV + g];
+    }
+    a.own_out[(g + NV0) * ld + i] = sweep_result(a.upper != 0, own, df, dg);
+}
+
+// SYS: 0 mean flow, 1 turbulence, 2 both (blockIdx.y picks the system).  a.lam
+// is the system's spectral radius; with SYS == 2 tlam is the turbulence one.
+template <int NV, int NFV, int NDIMS, int SYS, int GF>
+__global__ void __launch_bounds__(64) scalar_sweep_lanes_kernel(ScalarSweepArgs<double> a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ double sm[64 / (2 * GF) * GF * NFV];
+    if constexpr (SYS == 2) {
+        if (blockIdx.y == 1) {
+            a.lam = a.tlam;
+            scalar_sweep_lanes<NV, NFV, NDIMS, true, GF>(a, sm);
+            return;
+        }
+    }
+    scalar_sweep_lanes<NV, NFV, NDIMS, SYS == 1, GF>(a, sm);
 }
 
 // One level of both systems' sweeps, one thread per cell.  The builds

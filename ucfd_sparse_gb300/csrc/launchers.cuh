@@ -116,14 +116,59 @@ static void sweep_both_go(const ::ucfd::ScalarSweepArgs<T> &a, int block, cudaSt
         scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 1><<<grid_for(n, block), block, 0, s>>>(a);
 }
 
+// FP64 levels of at most this many cells take scalar_sweep_lanes_kernel: with
+// 4 / 8 pairs of lanes per cell.  One warp holds 4 / 2 cells and issues about
+// 95 FP64 instructions, against 480 (three active faces) to 900 (six) for a
+// warp of 32 cells with one thread per cell, so the lanes cost more pipe time
+// per cell and win while the sub-partitions (608) have few warps each.
+// Measured: natural-order FP64 step of 41x36x33 cells (108 levels of at most
+// 1100 cells, three active faces) 4.04 ms with one thread per cell in
+// blocks of 32, 0.91 ms with lanes chained by dependent launches.
+constexpr int kLanesCells4 = 12288, kLanesCells8 = 6144;
+
+template <int NV, int NFV, int NDIMS, int SYS>
+static void sweep_lanes_go(const ::ucfd::ScalarSweepArgs<double> &a, int gf, cudaStream_t s) {
+    const long long n = a.t1 - a.t0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_for(n * 2 * gf, 32), SYS == 2 ? 2 : 1);
+    cfg.blockDim = dim3(32);
+    cfg.stream = s;
+    // the next level's launch may start while this level runs
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.chained ? 1 : 0;
+    if (gf == 4) UCFD_CUDA(cudaLaunchKernelEx(&cfg, scalar_sweep_lanes_kernel<NV, NFV, NDIMS, SYS, 4>, a));
+    else UCFD_CUDA(cudaLaunchKernelEx(&cfg, scalar_sweep_lanes_kernel<NV, NFV, NDIMS, SYS, 8>, a));
+}
+
+// Pairs of lanes per cell for a level of this kind, 0: one thread per cell.
+static int sweep_lanes(const ::ucfd::ScalarSweepArgs<double> &a) {
+    const long long n = a.t1 - a.t0;
+    if (a.pair || a.facelist || a.nface > 8 || n <= 0) return 0;
+    const int most = a.max_active > 0 ? a.max_active : a.nface;
+    if (most <= 4) return n <= kLanesCells4 ? 4 : 0;
+    return n <= kLanesCells8 ? 8 : 0;
+}
+static int sweep_lanes(const ::ucfd::ScalarSweepArgs<float> &) { return 0; }
+
 // rans: 0 mean-flow system, 1 turbulence system, 2 both in one launch.
 template <typename T>
 void scalar_sweep(const ::ucfd::ScalarSweepArgs<T> &a, int nv, int nfv, int ndims, int rans,
                   int block, cudaStream_t s) {
     if (a.facelist) block = block > 0 ? block : kBlock;
     else block = spread_block<T>(a.pair ? 2ll * (a.t1 - a.t0) : a.t1 - a.t0, block);
+    const int gf = sweep_lanes(a);
 #define UCFD_SW(NV, NFV, ND)                                                   \
     if (nv == NV && nfv == NFV && ndims == ND) {                               \
+        if constexpr (sizeof(T) == 8) {                                        \
+            if (gf > 0 && rans == 0) return sweep_lanes_go<NV, NFV, ND, 0>(a, gf, s); \
+            if constexpr (NV > NFV) {                                          \
+                if (gf > 0 && rans == 1) return sweep_lanes_go<NV, NFV, ND, 1>(a, gf, s); \
+                if (gf > 0) return sweep_lanes_go<NV, NFV, ND, 2>(a, gf, s);   \
+            }                                                                  \
+        }                                                                      \
         if (rans == 2) {                                                       \
             if constexpr (NV > NFV) return sweep_both_go<T, NV, NFV, ND>(a, block, s); \
         } else if (rans) {                                                     \

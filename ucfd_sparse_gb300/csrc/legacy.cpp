@@ -118,8 +118,9 @@ void serial_schedule(LegacyCtx &c, int neles, int nface, const int *nei, cudaStr
 void launch_sweep(LegacyCtx &c, bool upper, bool rans, int t0, int t1, int neles, int nface, const int *nei,
                   const int *cells, const int *lcolor, const double *fnv, const double *vec, const double *upts,
                   const double *nbsrc, const double *own_in, double *own_out, const double *diag,
-                  const double *fspr, cudaStream_t s) {
+                  const double *fspr, bool chained, cudaStream_t s) {
     ScalarSweepArgs<double> a{};
+    a.chained = chained ? 1 : 0;  // the previous launch is the previous level of this sweep
     a.t0 = t0;
     a.t1 = t1;
     a.cells = cells;
@@ -185,13 +186,13 @@ void sweep(bool serial, bool upper, bool rans, bool inplace, int n0, int ne, int
             const int l = upper ? c.nlev - 1 - q : q;
             launch_sweep(c, upper, rans, c.lev_off[l], c.lev_off[l + 1], neles, nface, a_nei.dev, c.d_perm.p,
                          c.d_level.p, a_fnv.dev, a_vec.dev, a_upts.dev, nbsrc, own_in, own_out, a_diag.dev,
-                         a_fspr.dev, s);
+                         a_fspr.dev, q > 0, s);
         }
     } else {
         auto a_ic = stage<int>(icolor, N, c.s_icolor, s);
         auto a_lc = stage<int>(lcolor, N, c.s_lcolor, s);
         launch_sweep(c, upper, rans, n0, ne, neles, nface, a_nei.dev, a_ic.dev, a_lc.dev, a_fnv.dev, a_vec.dev,
-                     a_upts.dev, nbsrc, own_in, own_out, a_diag.dev, a_fspr.dev, s);
+                     a_upts.dev, nbsrc, own_in, own_out, a_diag.dev, a_fspr.dev, false, s);
     }
     writeback(upper && !inplace ? a_rhs : a_dub, s);
     done(s);
