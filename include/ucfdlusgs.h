@@ -115,13 +115,12 @@ UCFD_EXTERN ucfd_status_t UCFDFlowSysSetLaunch(FlowSys sys, int threads_per_bloc
  * No counterpart in the reference (its launch shape is the compile-time
  * TPB/BLOCK macro of Makefile.inc). */
 typedef struct {
-    int threads_per_block; /* sweep kernels: 0 (default 256) or 32..256 step 32 */
+    int threads_per_block; /* sweep kernels: most threads per block, 32..256 step 32 (small levels
+                              take fewer); 0: chosen by the size of the level */
     int sweep_variant;     /* block sweep: 0 faces unrolled to the ELL width, 1 face loop,
                               2 / 3 FP32 5x5 with J and LU tiles staged in shared memory
                               by bulk copies (2 / 1 buffers per warp; ELL width 6 or 4),
-                              4 = 0 launched as a programmatic dependent of the previous
-                              colour (its start overlaps the previous colour's tail);
-                              5 = 0 for the block sweep;
+                              4 and 5 = 0 for the block sweep;
                               scalar sweeps: 0 default build, 1 / 2 capped at 80 / 64
                               registers (more resident warps), 3 / 4 two threads per
                               cell, 5 one thread per active face (per-level launches;

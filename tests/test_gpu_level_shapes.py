@@ -24,3 +24,50 @@ def test_scalar_levels_either_side_of_the_lane_kernel(m, port, ucfd):
     cl.colored_step(d, dev(icolor), ranges, diag, torch.zeros_like(d["rhs"]))
     ref = port.legacy_step(c, icolor, ranges, c["lcolor"])[0]
     np.testing.assert_array_equal(d["upts"].cpu().numpy(), ref)
+
+
+# checkerboard colours of 32, 7812/7813 (a lane per block row) and 8788 cells
+# (one thread per cell): either side of the FP64 kernels' boundary at 8192
+@pytest.mark.parametrize("m", [4, 25, 26])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_block_levels_and_kept_terms(m, prec, ucfd):
+    """A sweep that reads the other side's terms or sums from the sweep before
+    equals one that forms every face itself (Prepare before each sweep makes
+    the kept ones stale), bit for bit, in any order of sweeps and with a
+    Reset in between."""
+    from tests.test_gpu_blusgs import make
+    b = mg.blusgs_case(m, permute=False, seed=m)
+    c = np.arange(m ** 3)
+    color = ((c % m + c // m % m + c // (m * m)) & 1).astype(np.int32)
+    got = []
+    for stale in (False, True):
+        S, e = make(b, prec=prec, on_device=True, colored=color)
+        S.blusgs_pack(0, 0.0)
+        S.blusgs_ns_prepare()
+        S.blusgs_reset()
+        for step in "luluullRluul":
+            if step == "R":
+                S.blusgs_reset()
+                continue
+            if stale:
+                S.blusgs_ns_prepare()
+            (S.blusgs_ns_lower if step == "l" else S.blusgs_ns_upper)()
+        S.blusgs_update(0)
+        got.append(e["upts"].cpu().numpy())
+    np.testing.assert_array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("m", [25, 26])
+def test_block_levels_match_the_oracle(m, port, ucfd):
+    from tests.test_gpu_blusgs import host, make, run_sweeps
+    b = mg.blusgs_case(m, seed=m)
+    from ucfd_sparse_gb300 import coloredlusgs as cl
+    ic, rg, lc = cl.greedy_coloring_csr(b["rowptr"], b["colidx"])
+    S, e = make(b, colored=lc)
+    run_sweeps(S, 2)
+    new = np.empty(b["nlocal"], dtype=np.int64)
+    new[ic] = np.arange(b["nlocal"])
+    br = mg.renumber_flowsys(b, new)
+    up, _, res, _ = port.flowsys_blusgs(br, b["rhs"], b["dt"], b["jmat"], b["vol"], b["upts"], nsweeps=2)
+    np.testing.assert_array_equal(host(e["upts"]), up)
+    np.testing.assert_array_equal(host(e["res"]), res)

@@ -40,12 +40,12 @@ struct Work {
     DevBuf<S> fl_geo[2];                   // face lists (lower, upper): normal + fa * rv per entry
     DevBuf<S> ulo;                         // FP32 mode: low part of the float-float state u + ulo (UCFDLUSGS_Run)
     DevBuf<S> crhs;                        // fast modes: D^-1 rhs, the block sweeps' right-hand side
-    DevBuf<S> spart;                       // fast modes: each block sweep's own-side sums (SweepSplit)
+    DevBuf<S> spart;                       // each block sweep's own-side sums or terms (SweepSplit)
     DevBuf<float4> geo4;                   // FP32 run loop with both systems: (normal, fa * rv) per cell-face
     DevBuf<float2> lam2;                   // and (lam, tlam) per cell-face
 };
 
-// Which increments the fast block sweeps' stored sums (Work::spart) belong
+// Which increments the block sweeps' stored sums or terms (Work::spart) belong
 // to: the sweeps into du in direction dir (0 lower, 1 upper) with the
 // blocks of Prepare number ver.  The next sweep in the other direction
 // into the same du reads them instead of forming that side again.
@@ -85,6 +85,7 @@ struct _FlowSys {
     DevBuf<int> d_iperm, d_nei, d_slot;
     DevBuf<int8_t> d_side;
     DevBuf<double> fa64, rv64;
+    DevBuf<double> fv64;  // FP64 modes: face area * rcp_vol per cell-face, the product the sweeps form
 
     Work<double> w64;
     Work<float> w32;
@@ -98,7 +99,7 @@ struct _FlowSys {
     SplitState split[2];           // NS / turbulence rows of the fast block sweeps
     unsigned jver[2] = {1, 1};     // Prepare count of the NS / turbulence blocks
     bool has_self = false;         // some CSR row lists itself
-    std::vector<int> act[2];       // per level: most faces of a cell towards earlier / later levels
+    std::vector<int> act[2];       // per level: most faces of a cell towards earlier / later levels (0: not known)
     bool lam2_ok = false;          // Work::lam2 packs the current NS and RANS spectral radii (FP32)
     DevBuf<double> part, red, resid;
     PinnedBuf<double> h_red;
@@ -124,6 +125,10 @@ void finish(FlowSys s, bool force_sync = false) {
     UCFD_CHECK_LAUNCH();
     if (!s->async || force_sync) UCFD_CUDA(cudaStreamSynchronize(s->stream()));
 }
+
+// Largest level whose active faces are counted on the host (scalar sweeps of
+// larger levels do not ask).
+constexpr int kActLevel = 16384;
 
 // Build the level schedule and the ELL mesh arrays (once).
 void build_topology(FlowSys s) {
@@ -173,18 +178,6 @@ void build_topology(FlowSys s) {
         sort_levels_by(s->sch, bfs);
     }
     const Schedule &sch = s->sch;
-    for (std::vector<int> &v : s->act) v.assign(sch.nlev, 0);
-    for (int l = 0; l < sch.nlev; ++l)
-        for (int k = sch.lev_off[l]; k < sch.lev_off[l + 1]; ++k) {
-            int n0 = 0, n1 = 0;
-            for (int q = rp[sch.perm[k]]; q < rp[sch.perm[k] + 1]; ++q) {
-                const int nb = sch.iperm[ci[q]];
-                n0 += nb < sch.lev_off[l];
-                n1 += nb >= sch.lev_off[l + 1];
-            }
-            s->act[0][l] = std::max(s->act[0][l], n0);
-            s->act[1][l] = std::max(s->act[1][l], n1);
-        }
     int P = 0;
     for (int i = 0; i < n; ++i) P = std::max(P, rp[i + 1] - rp[i]);
     P = std::max(P, 1);
@@ -207,6 +200,23 @@ void build_topology(FlowSys s) {
                 enrm[(p * s->ndims + d) * N + k] = sd[q] * fn[sl[q] + (size_t)d * s->nfaces];
         }
     }
+    // small levels (the ones whose FP64 scalar sweeps ask): the most faces of
+    // a cell towards earlier / later levels
+    for (std::vector<int> &v : s->act) v.assign(sch.nlev, 0);
+    for (int l = 0; l < sch.nlev && s->prec != UCFD_PREC_FP32; ++l) {
+        const int k0 = sch.lev_off[l], k1 = sch.lev_off[l + 1];
+        if (k1 - k0 > kActLevel) continue;
+        for (int k = k0; k < k1; ++k) {
+            int n0 = 0, n1 = 0;
+            for (int p = 0; p < P; ++p) {
+                const int nb = nei[p * N + k];
+                n0 += nb >= 0 && nb < k0;
+                n1 += nb >= k1;
+            }
+            s->act[0][l] = std::max(s->act[0][l], n0);
+            s->act[1][l] = std::max(s->act[1][l], n1);
+        }
+    }
     cudaStream_t st = s->stream();
     s->d_iperm.upload(sch.iperm.data(), N, st);
     s->d_nei.upload(nei.data(), nei.size(), st);
@@ -215,6 +225,10 @@ void build_topology(FlowSys s) {
     s->fa64.upload(efa.data(), efa.size(), st);
     s->rv64.upload(erv.data(), erv.size(), st);
     s->w64.nrm.upload(enrm.data(), enrm.size(), st);
+    if (s->prec != UCFD_PREC_FP32) {
+        s->fv64.ensure((size_t)P * N);
+        kfast::face_fv(N, P, s->fa64.p, s->rv64.p, s->fv64.p, st);
+    }
     if (s->prec == UCFD_PREC_FP32) {
         std::vector<float> f(efa.begin(), efa.end());
         s->w32.fa.upload(f.data(), f.size(), st);
@@ -400,7 +414,7 @@ void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent =
         a.t1 = s->sch.lev_off[l + 1];
         a.lo = a.t0;
         a.hi = a.t1;
-        a.max_active = std::max(s->act[upper ? 1 : 0][l], 1);
+        a.max_active = s->act[upper ? 1 : 0][l];
         a.chained = launched;
         launched = launched || a.t1 > a.t0;
         KCALL(EX, scalar_sweep<S>, a, s->nvars, s->nfvars, s->ndims, sys, s->block, s->stream());
@@ -502,26 +516,27 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     const int B = turb ? s->ntvars : s->nfvars;
     const int var0 = turb ? s->nfvars : 0;
     const int L = s->sch.nlev;
+    // partial when the stored sums (exact mode: terms) are the previous
+    // opposite sweep's into the same du with the same blocks (a face to the
+    // cell itself changes with the cell's own increment: such meshes always
+    // sweep in full mode)
     SweepSplit<S> sp;
-    if constexpr (!EX) {
-        // the fast build's split sums: partial when the stored sums are the
-        // previous opposite sweep's into the same du with the same blocks
-        SplitState &ss = s->split[turb ? 1 : 0];
-        sp.part = w.spart.ensure((size_t)s->nvars * s->N);
-        sp.upper = upper ? 1 : 0;
-        // (a face to the cell itself changes with the cell's own increment:
-        // such meshes always sweep in full mode)
-        sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0])
-                      ? 0 : 1;
-    }
+    SplitState &ss = s->split[turb ? 1 : 0];
+    sp.part = w.spart.ensure((size_t)(EX ? s->P : 1) * s->nvars * s->N);
+    sp.upper = upper ? 1 : 0;
+    sp.nvars = s->nvars;
+    sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0]) ? 0 : 1;
+    const S *fa = geo_fa<S>(s);
+    if constexpr (EX) fa = s->fv64.p;
     if (s->variant == 2 || s->variant == 3) s->bulk_swept = true;
     for (int q = 0; q < L; ++q) {
         const int l = upper ? L - 1 - q : q;
         KCALL(EX, fs_blusgs_sweep<S>, B, s->sch.lev_off[l], s->sch.lev_off[l + 1], s->N, s->P, var0,
-              s->d_nei.p, geo_fa<S>(s), geo_rv<S>(s), turb ? w.tJ.p : w.J.p, blu_LU<S>(s, turb), rhs, du,
+              s->d_nei.p, fa, geo_rv<S>(s), turb ? w.tJ.p : w.J.p, blu_LU<S>(s, turb), rhs, du,
               s->block, s->variant, s->d_sweep_err.p, kBulkMaxSpin, sp, s->stream());
+        if (s->sch.lev_off[l + 1] > s->sch.lev_off[l]) sp.chained = 1;
     }
-    if constexpr (!EX) s->split[turb ? 1 : 0] = SplitState{du, upper ? 1 : 0, s->jver[turb ? 1 : 0]};
+    ss = SplitState{du, upper ? 1 : 0, s->jver[turb ? 1 : 0]};
 }
 
 // du of the fast block sweeps was set to zero: both sides' sums are zero,
@@ -927,7 +942,7 @@ ucfd_status_t UCFDFlowSysAutotune(FlowSys s, int reps, UCFDLaunchConfig *best) {
             };
             // the unrolled kernels exist for ELL widths 6 and 4 only
             const bool unrolled = s->P == 6 || s->P == 4;
-            for (int v : {0, 1, 4}) {
+            for (int v : {0, 1}) {  // 4 is 0: both chain the levels' launches
                 if (v != 0 && !unrolled) continue;
                 for (int b : kTuneBlocks) {
                     s->block = b;
@@ -1358,6 +1373,8 @@ ucfd_status_t UCFDBLUSGS_Reset(FlowSys s) {
         if constexpr (!EX) {
             split_zero<S>(s, false, w.bdu.p, st);
             if (s->ntvars > 0) split_zero<S>(s, true, w.bdu.p, st);
+        } else {
+            split_forget(s);  // the next sweep forms every term of the zero increments itself
         }
     });
     s->du64_valid = false;

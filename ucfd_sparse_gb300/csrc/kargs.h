@@ -76,22 +76,27 @@ struct ScalarSweepArgs {
     const T *fl_geo;       // [E][4] outward normal (zero-padded to 3 components) and fa * rv
 };
 
-// Block LU-SGS sweeps of the fast build (M = D^-1 J fv blocks): a cell's
-// face products are summed by the level of the neighbour -- S_lo over
-// earlier levels, S_up over later ones -- and du = c - S_lo - S_up.  A
-// lower sweep reaches a cell after every earlier level and before every
-// later one, an upper sweep the other way round, so the side a sweep does
-// not update is the sum the previous (opposite) sweep formed with the same
+// Block LU-SGS sweeps form only one side of a cell's faces.  A lower sweep
+// reaches a cell after every earlier level and before every later one, an
+// upper sweep the other way round, so what the side a sweep does not update
+// contributes is what the previous (opposite) sweep formed with the same
 // increments.  part keeps each sweep's own side for the next one; with
-// full == 0 a sweep reads the other side from part instead of loading
-// those faces again.  Either way the values are the same, bit for bit.
-// (A face to the cell itself goes with the other side's sum; a mesh with
-// such faces always sweeps in full mode.)
+// full == 0 a sweep reads the other side from part instead of loading and
+// multiplying those blocks again.  Either way the values are the same, bit
+// for bit.
+//   Fast build (M = D^-1 J fv blocks): one sum per side, S_lo and S_up, and
+//     du = c - S_lo - S_up; part [nvars][N].
+//   Exact build: the reference subtracts the faces one by one in face order,
+//     so each face's rounded term is kept; part [P][nvars][N].
+// (A face to the cell itself is formed by every sweep; a mesh with such
+// faces always sweeps in full mode.)
 template <typename S>
 struct SweepSplit {
-    S *part = nullptr;  // [nvars][N] sums of the sweep's own side (nullptr: exact build, no split)
+    S *part = nullptr;
     int upper = 0;      // this sweep's direction
     int full = 1;       // 1: form both sides; 0: the other side from part
+    int nvars = 0;      // rows of part per face (exact build)
+    int chained = 0;    // 1: the previous launch on the stream is the previous level of this sweep
 };
 
 // One colour of a transposed (adjoint) colored LU-SGS sweep.

@@ -358,7 +358,7 @@ __global__ void fs_blusgs_rhs_solve_kernel(long long N, int var0, const S *LU, c
     for (int r = 0; r < B; ++r) c[(var0 + r) * N + k] = v[r];
 }
 
-// ---- split sums of the fast build's sweeps (see SweepSplit in kargs.h) ----
+// ---- split sides of the sweeps (see SweepSplit in kargs.h) ----
 template <typename S>
 using SweepSplit = ::ucfd::SweepSplit<S>;
 
@@ -438,27 +438,29 @@ __device__ __forceinline__ void split_finish(const SweepSplit<S> &sp, long long 
 // J and LU tiles, rhs, nei, fa) and is loaded with the streaming
 // (evict-first) policy, so that du, gathered at every neighbour, keeps L2.
 //
-// DEP (PW > 0 only): launched as a programmatic dependent of the previous
-// sweep launch (one colour after the other).  The grid lets its own
-// dependent start at once, then loads every input the previous launch
-// does not write (rhs, rv, nei, fa) before it waits for that launch to
-// complete (griddepcontrol.wait); the neighbour increments du are read
-// after the wait.  This overlaps a launch's start with the previous
-// launch's tail, which pays where levels are small.  Results are those of
-// DEP == false.  (An L2 bulk prefetch of each warp's J and LU tiles in
-// front of the wait measured slower at 2.1M cells: the early grids'
-// prefetches evict the running grid's data.)
+// The unrolled form (PW > 0) is launched as a programmatic dependent of the
+// previous level's launch (sp.chained; one colour after the other).  The
+// grid lets its own dependent start at once, then loads every input the
+// previous level does not write (rhs, nei) before it waits for that launch
+// to complete (griddepcontrol.wait); the neighbour increments du are read
+// after the wait.  This overlaps a launch's start with the previous launch's
+// tail, which pays where levels are small (FP32 pair at 2.1M cells 0.396 ->
+// 0.354 ms).  The first level of a sweep is launched without the attribute,
+// so it starts after everything before the sweep.  (An L2 bulk prefetch of
+// each warp's J and LU tiles in front of the wait measured slower at 2.1M
+// cells: the early grids' prefetches evict the running grid's data.)
 //
 // Fast build (kFold): the face products are split by side (split_add /
 // split_finish; SweepSplit in kargs.h).  In partial mode the faces of the
-// other side are neither loaded nor multiplied.
-template <typename S, int B, int PW, bool DEP = false>
+// other side are neither loaded nor multiplied.  The exact build keeps the
+// faces' terms instead of sums: FP64 instructions bound it (one per 64 clocks
+// and SM sub-partition), and a stored term replaces 55 of them by 5.
+template <typename S, int B, int PW>
 __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, long long N, int P,
                                                               int var0, const int *nei, const S *fa,
                                                               const S *rv, const S *J, const S *LU,
                                                               const S *rhs, S *du, SweepSplit<S> sp) {
-    static_assert(!DEP || PW > 0, "the dependent-launch form is the unrolled one");
-    if constexpr (DEP) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (PW > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // threads start at the tile boundary below t0, so every warp reads
     // whole tiles; the cells of the tile outside [t0, t1) do nothing
     const int k = (t0 & ~31) + blockIdx.x * blockDim.x + threadIdx.x;
@@ -470,7 +472,7 @@ __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, lo
     for (int r = 0; r < B; ++r) b[r] = __ldcs(rhs + (var0 + r) * N + k);
     if constexpr (kFold) {
         S ta[B], to[B];
-        if constexpr (!DEP) split_start<S, B>(sp, N, var0, k, ta, to);
+        if constexpr (PW == 0) split_start<S, B>(sp, N, var0, k, ta, to);
         if constexpr (PW > 0) {
             // the faces the sweep uses, as bits (own: those of its own side)
             int nb[PW];
@@ -482,10 +484,8 @@ __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, lo
                 use |= (sd >= 0 && split_uses(sp, sd)) ? 1u << p : 0u;
                 own |= (sd == sp.upper) ? 1u << p : 0u;
             }
-            if constexpr (DEP) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                split_start<S, B>(sp, N, var0, k, ta, to);
-            }
+            if (sp.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
+            split_start<S, B>(sp, N, var0, k, ta, to);
             // KB used faces at a time, in face order: the step's neighbour
             // increments are all requested before its products
             constexpr int KB = sizeof(S) == 8 ? 2 : 3;
@@ -537,56 +537,53 @@ __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, lo
         return;
     }
     // exact build: the reference's per-face products (blusgs.c:298-314),
-    // scaled by fv, then the LU solve of the diagonal block
-    const S rvk = rv[k];
+    // scaled by fv, subtracted in face order, then the LU solve of the
+    // diagonal block.  fa holds fv = face area * rcp_vol (the same product
+    // the reference forms per face).  One face: its term formed (used by
+    // this sweep) or read back (formed by the previous one).
+    const auto face = [&](int p, int g) {
+        S *term = sp.part + ((long long)p * sp.nvars + var0) * N + k;
+        const int sd = split_side(g, t0, t1);
+        if (!split_uses(sp, sd)) {
+            S v[B];
+#pragma unroll
+            for (int r = 0; r < B; ++r) v[r] = __ldcs(term + r * N);
+#pragma unroll
+            for (int r = 0; r < B; ++r) b[r] -= v[r];
+            return;
+        }
+        S x[B];
+#pragma unroll
+        for (int c = 0; c < B; ++c) x[c] = du[(var0 + c) * N + g];
+        const S fv = __ldcs(fa + p * N + k);
+        const S *Jp = Jk + ((long long)p * B2 << 5);
+#pragma unroll
+        for (int r = 0; r < B; ++r) {
+            S val = __ldcs(Jp + ((r * B) << 5)) * x[0];
+#pragma unroll
+            for (int c = 1; c < B; ++c) val += __ldcs(Jp + ((r * B + c) << 5)) * x[c];
+            val *= fv;
+            b[r] -= val;
+            if (sd == sp.upper) term[r * N] = val;
+        }
+    };
     if constexpr (PW > 0) {
         int nb[PW];
-        S fv[PW];
 #pragma unroll
+        for (int p = 0; p < PW; ++p) nb[p] = __ldcs(nei + p * N + k);
+        if (sp.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll 1
         for (int p = 0; p < PW; ++p) {
-            nb[p] = __ldcs(nei + p * N + k);
-            fv[p] = __ldcs(fa + p * N + k) * rvk;
-        }
-        if constexpr (DEP) asm volatile("griddepcontrol.wait;" ::: "memory");
-        S x[PW][B];
+            int g = nb[0];
 #pragma unroll
-        for (int p = 0; p < PW; ++p) {
-            const int g = nb[p] >= 0 ? nb[p] : k;  // padding: any valid address
-#pragma unroll
-            for (int c = 0; c < B; ++c) x[p][c] = du[(var0 + c) * N + g];
-        }
-#pragma unroll
-        for (int p = 0; p < PW; ++p) {
-            const S *Jp = Jk + ((long long)p * B2 << 5);
-            S jv[B2];
-#pragma unroll
-            for (int e = 0; e < B2; ++e) jv[e] = __ldcs(Jp + (e << 5));
-            if (nb[p] >= 0) {
-#pragma unroll
-                for (int r = 0; r < B; ++r) {
-                    S val = S(0);
-#pragma unroll
-                    for (int c = 0; c < B; ++c) val += jv[r * B + c] * x[p][c];
-                    b[r] -= val * fv[p];
-                }
-            }
+            for (int q = 1; q < PW; ++q) g = q == p ? nb[q] : g;
+            if (g >= 0) face(p, g);
         }
     } else {
         for (int p = 0; p < P; ++p) {
-            const int nb = __ldcs(nei + p * N + k);
-            if (nb < 0) break;
-            const S fv = __ldcs(fa + p * N + k) * rvk;
-            S x[B];
-#pragma unroll
-            for (int c = 0; c < B; ++c) x[c] = du[(var0 + c) * N + nb];
-            const S *Jp = Jk + ((long long)p * B2 << 5);
-#pragma unroll
-            for (int r = 0; r < B; ++r) {
-                S val = S(0);
-#pragma unroll
-                for (int c = 0; c < B; ++c) val += __ldcs(Jp + ((r * B + c) << 5)) * x[c];
-                b[r] -= val * fv;
-            }
+            const int g = __ldcs(nei + p * N + k);
+            if (g < 0) break;
+            face(p, g);
         }
     }
     S lu[B2];
@@ -600,7 +597,7 @@ __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, lo
 
 // FP32 sweep of a small level (a colour of a few thousand cells), where a
 // launch costs one thread's chain of dependent memory round trips rather
-// than bandwidth.  Launched like the DEP form of fs_blusgs_sweep_kernel,
+// than bandwidth.  Launched like the unrolled fs_blusgs_sweep_kernel,
 // but every input the previous launch does not write -- rhs, nei and the
 // blocks of the faces the sweep uses -- is loaded into registers before
 // griddepcontrol.wait, so after the wait only the neighbour increments
@@ -630,7 +627,7 @@ __global__ void __launch_bounds__(128) fs_blusgs_sweep_small_kernel(int t0, int 
             for (int e = 0; e < B2; ++e) jv[p][e] = __ldcs(Jk + ((p * B2 + e) << 5));
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (sp.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
     float ta[B], to[B];
     split_start<float, B>(sp, N, var0, k, ta, to);
     float x[PW][B];
@@ -649,6 +646,123 @@ __global__ void __launch_bounds__(128) fs_blusgs_sweep_small_kernel(int t0, int 
     split_finish<float, B>(sp, N, var0, k, b, ta, to);
 #pragma unroll
     for (int r = 0; r < B; ++r) du[(var0 + r) * N + k] = b[r];
+}
+
+// FP64 sweep of a small level, B lanes per cell (lane r forms row r of every
+// product; 32 / B cells per warp).  With one thread per cell such a level
+// costs one thread's FP64 instructions at 64 clocks each (exact build about
+// 270 with half the faces kept, 420 without; fast build 90) and its serial
+// loads; a row's lane issues a fifth of the products, and everything the
+// previous level does not write (blocks, kept terms or sums, LU row, right-
+// hand side) is loaded before griddepcontrol.wait.  The LU solve passes each
+// solved value from lane to lane.  Each row's operations and their order are
+// those of fs_blusgs_sweep_kernel (a sum's leading 0 + x is dropped), so the
+// values are the same.
+template <int B, int PW>
+__global__ void __launch_bounds__(32) fs_blusgs_sweep_rows_kernel(int t0, int t1, long long N, int var0,
+                                                                  const int *nei, const double *fv,
+                                                                  const double *J, const double *LU,
+                                                                  const double *rhs, double *du,
+                                                                  SweepSplit<double> sp) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    constexpr int C = 32 / B, B2 = B * B;
+    const int lane = threadIdx.x, c = lane / B, r = lane - c * B, base = c * B;
+    const int kc = t0 + blockIdx.x * C + c;
+    const bool valid = c < C && kc < t1;
+    const long long k = valid ? kc : t0;  // idle lanes: any valid cell, nothing stored
+    const long long vk = (var0 + r) * N + k;
+    const double *Jr = J + ::ucfd::tile_index(k, r * B, (long long)PW * B2);
+    double b = __ldcs(rhs + vk);
+    double jv[PW][B], f[PW], kept[PW], lu[B], lud = 1.0;
+    int nb[PW];
+    unsigned use = 0u, own = 0u;
+#pragma unroll
+    for (int p = 0; p < PW; ++p) {
+        nb[p] = __ldg(nei + p * N + k);
+        const int sd = nb[p] >= 0 ? split_side(nb[p], t0, t1) : -1;
+        const bool u = sd >= 0 && split_uses(sp, sd);
+        use |= u ? 1u << p : 0u;
+        own |= sd == sp.upper ? 1u << p : 0u;
+        if (u) {
+#pragma unroll
+            for (int q = 0; q < B; ++q) jv[p][q] = __ldcs(Jr + ((p * B2 + q) << 5));
+            if constexpr (!kFold) f[p] = __ldg(fv + p * N + k);
+        } else if (!kFold && sd >= 0) {
+            kept[p] = sp.part[((long long)p * sp.nvars + var0 + r) * N + k];
+        }
+    }
+    double to = 0.0;
+    if constexpr (kFold) {
+        if (!sp.full) to = sp.part[vk];
+    } else {
+        const double *LUr = LU + ::ucfd::tile_index(k, r * B, B2);
+#pragma unroll
+        for (int q = 0; q < B; ++q) lu[q] = __ldg(LUr + (q << 5));
+        lud = __ldg(LUr + (r << 5));
+    }
+    if (sp.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
+    double x[PW][B];
+#pragma unroll
+    for (int p = 0; p < PW; ++p) {
+        if ((use >> p) & 1u) {
+#pragma unroll
+            for (int q = 0; q < B; ++q) x[p][q] = __ldcg(du + (var0 + q) * N + nb[p]);
+        }
+    }
+    if constexpr (kFold) {
+        double ta = 0.0;
+#pragma unroll
+        for (int p = 0; p < PW; ++p) {
+            if ((use >> p) & 1u) {
+                double t = (own >> p) & 1u ? ta : to;
+#pragma unroll
+                for (int q = 0; q < B; ++q) t = fma(jv[p][q], x[p][q], t);
+                if ((own >> p) & 1u) ta = t;
+                else to = t;
+            }
+        }
+        b = (b - (sp.upper ? to : ta)) - (sp.upper ? ta : to);
+        if (valid) {
+            sp.part[vk] = ta;
+            du[vk] = b;
+        }
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < PW; ++p) {
+        if ((use >> p) & 1u) {
+            double val = jv[p][0] * x[p][0];
+#pragma unroll
+            for (int q = 1; q < B; ++q) val += jv[p][q] * x[p][q];
+            val *= f[p];
+            b -= val;
+            if (valid && (own >> p) & 1u) sp.part[((long long)p * sp.nvars + var0 + r) * N + k] = val;
+        } else if (nb[p] >= 0) {
+            b -= kept[p];
+        }
+    }
+    // lusub (inverse.h:51-80): row r subtracts its sum once every earlier
+    // (later) value is final; the upper sums go in column order
+    double v = 0.0, pr[B];
+#pragma unroll
+    for (int q = 0; q < B - 1; ++q) {
+        const double bq = __shfl_sync(0xffffffffu, b, base + q);
+        if (r > q) v = q == 0 ? lu[0] * bq : v + lu[q] * bq;
+        if (r == q + 1) b -= v;
+    }
+    if (r == B - 1) b /= lud;
+#pragma unroll
+    for (int q = B - 1; q > 0; --q) {
+        const double bq = __shfl_sync(0xffffffffu, b, base + q);
+        pr[q] = lu[q] * bq;
+        if (r == q - 1) {
+            double t = pr[q];  // r + 1 == q: the row's first column
+#pragma unroll
+            for (int s = q + 1; s < B; ++s) t += pr[s];
+            b = (b - t) / lud;
+        }
+    }
+    if (valid) du[vk] = b;
 }
 
 // FP32 block sweep with each tile's J and LU staged in shared memory by

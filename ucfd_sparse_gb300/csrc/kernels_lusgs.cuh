@@ -763,6 +763,13 @@ __global__ void face_list_geo_kernel(long long E, long long ld, int ndims, const
     }
 }
 
+// fv = face area * rcp_vol per cell-face.
+__global__ void face_fv_kernel(long long N, int P, const double *fa, const double *rv, double *fv) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)P * N;
+         e += (long long)gridDim.x * blockDim.x)
+        fv[e] = fa[e] * rv[e % N];
+}
+
 // Packed geometry of the FP32 run loop with both systems, per cell-face
 // (p, k): (outward normal, zero-padded to 3 components; fa * rv).
 __global__ void pack_geo4_kernel(long long N, int P, int ndims, const float *nrm, const float *fa, const float *rv,

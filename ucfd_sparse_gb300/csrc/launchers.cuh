@@ -56,6 +56,13 @@ void face_list_geo(long long E, long long ld, int ndims, const int *q, const T *
                                                                                           rv, geo);
 }
 
+void face_fv(long long N, int P, const double *fa, const double *rv, double *fv, cudaStream_t s) {
+    const long long n = (long long)P * N;
+    if (n <= 0) return;
+    const long long g = (n + kBlock - 1) / kBlock;
+    face_fv_kernel<<<(unsigned)(g < 65535 * 16 ? g : 65535 * 16), kBlock, 0, s>>>(N, P, fa, rv, fv);
+}
+
 void pack_geo4(long long N, int P, int ndims, const float *nrm, const float *fa, const float *rv, void *geo4,
                cudaStream_t s) {
     const long long n = (long long)P * N;
@@ -385,8 +392,12 @@ static void sweep_bulk_go(int t0, int t1, long long N, int var0, const int *nei,
     kern<<<g, threads, smem, s>>>(t0, t1, N, var0, nei, fa, rv, J, LU, rhs, du, err, max_spin, sp);
 }
 
-// Unrolled sweep launched as a programmatic dependent of the previous
-// launch on the stream (cudaLaunchAttributeProgrammaticStreamSerialization).
+// Unrolled sweep; in FP32 launched as a programmatic dependent of the
+// previous level's launch (cudaLaunchAttributeProgrammaticStreamSerialization).
+// In FP64 not: the waiting blocks crowd onto the SMs that run out of work
+// first, and the FP64 pipe of those few SMs then bounds the level (226K cells,
+// exact build: pair 510 us dependent, 389 us not; FMA 167 and 166 us; FP32
+// 83 and 95 us).
 template <typename S, int B, int PW>
 static void sweep_dep_go(unsigned g, int block, cudaStream_t s, int t0, int t1, long long N, int P, int var0,
                          const int *nei, const S *fa, const S *rv, const S *J, const S *LU, const S *rhs, S *du,
@@ -400,14 +411,15 @@ static void sweep_dep_go(unsigned g, int block, cudaStream_t s, int t0, int t1, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    UCFD_CUDA(cudaLaunchKernelEx(&cfg, fs_blusgs_sweep_kernel<S, B, PW, true>, t0, t1, N, P, var0, nei, fa, rv, J,
-                                 LU, rhs, du, sp));
+    ::ucfd::SweepSplit<S> q = sp;
+    if (std::is_same<S, double>::value) q.chained = 0;
+    cfg.numAttrs = q.chained ? 1 : 0;
+    UCFD_CUDA(cudaLaunchKernelEx(&cfg, fs_blusgs_sweep_kernel<S, B, PW>, t0, t1, N, P, var0, nei, fa, rv, J,
+                                 LU, rhs, du, q));
 }
 
-// Levels with at most this many cells take the register-hoisted kernel in
-// the dependent-launch variant (FP32): they are bound by one thread's
-// memory latency, not by bandwidth.
+// FP32 levels with at most this many cells take the register-hoisted kernel:
+// they are bound by one thread's memory latency, not by bandwidth.
 constexpr int kSmallLevel = 16384;
 
 template <int B, int PW>
@@ -423,8 +435,30 @@ static void sweep_small_go(cudaStream_t s, int t0, int t1, long long N, int var0
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = sp.chained ? 1 : 0;
     UCFD_CUDA(cudaLaunchKernelEx(&cfg, fs_blusgs_sweep_small_kernel<B, PW>, t0, t1, N, var0, nei, J, rhs, du, sp));
+}
+
+// FP64 levels of at most this many cells take the kernel with B lanes per
+// cell: a warp then holds 32 / B cells and costs about 60 FP64 instructions
+// (fast build 32), against 270-420 (90) for 32 cells with one thread each.
+constexpr int kRowsCells = 8192;
+
+template <int B, int PW>
+static void sweep_rows_go(cudaStream_t s, int t0, int t1, long long N, int var0, const int *nei, const double *fv,
+                          const double *J, const double *LU, const double *rhs, double *du,
+                          const ::ucfd::SweepSplit<double> &sp) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_for(t1 - t0, 32 / B));
+    cfg.blockDim = dim3(32);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = sp.chained ? 1 : 0;
+    UCFD_CUDA(cudaLaunchKernelEx(&cfg, fs_blusgs_sweep_rows_kernel<B, PW>, t0, t1, N, var0, nei, fv, J, LU, rhs, du,
+                                 sp));
 }
 
 template <typename S>
@@ -436,27 +470,22 @@ void fs_blusgs_sweep(int B, int t0, int t1, long long N, int P, int var0, const 
     block = spread_block<S>(t1 - t0, block);
     // threads start at the tile boundary below t0 (see the kernel)
     const unsigned g = grid_for(t1 - (t0 & ~31), block);
-    // variant 0: faces unrolled to the ELL width (6 or 4) when it matches;
+    // variants 0 and 4: faces unrolled to the ELL width (6 or 4) when it
+    // matches, each level a programmatic dependent launch of the previous;
     // variant 1: the face loop that stops at the first padding slot;
     // variants 2 / 3: FP32, ELL width 6 or 4, block 5: J and LU tiles staged
-    // in shared memory by bulk copies, 2 / 1 buffers per warp;
-    // variant 4: variant 0 launched as a programmatic dependent of the
-    // previous launch (its start overlaps the previous colour's tail).
+    // in shared memory by bulk copies, 2 / 1 buffers per warp.
     // All apply the faces in the same order with the same operations.
-    if (variant == 4 && (P == 6 || P == 4)) {
-        if constexpr (std::is_same<S, float>::value) {
-            if (kFold && B == 5 && t1 - t0 <= kSmallLevel) {
-                if (P == 6) sweep_small_go<5, 6>(s, t0, t1, N, var0, nei, J, rhs, du, sp);
-                else sweep_small_go<5, 4>(s, t0, t1, N, var0, nei, J, rhs, du, sp);
-                return;
+    if constexpr (std::is_same<S, double>::value) {
+        // small levels, whatever the variant
+        if (B > 1 && t1 - t0 <= kRowsCells && (P == 6 || P == 4)) {
+            if (P == 6) {
+                UCFD_BSW(B, (sweep_rows_go<BB, 6>(s, t0, t1, N, var0, nei, fa, J, LU, rhs, du, sp)));
+            } else {
+                UCFD_BSW(B, (sweep_rows_go<BB, 4>(s, t0, t1, N, var0, nei, fa, J, LU, rhs, du, sp)));
             }
+            return;
         }
-        if (P == 6) {
-            UCFD_BSW(B, (sweep_dep_go<S, BB, 6>(g, block, s, t0, t1, N, P, var0, nei, fa, rv, J, LU, rhs, du, sp)));
-        } else {
-            UCFD_BSW(B, (sweep_dep_go<S, BB, 4>(g, block, s, t0, t1, N, P, var0, nei, fa, rv, J, LU, rhs, du, sp)));
-        }
-        return;
     }
     if constexpr (std::is_same<S, float>::value) {
         if ((variant == 2 || variant == 3) && B == 5 && (P == 6 || P == 4)) {
@@ -471,19 +500,23 @@ void fs_blusgs_sweep(int B, int t0, int t1, long long N, int P, int var0, const 
             return;
         }
     }
-    if (variant == 1) {
-        UCFD_BSW(B, (fs_blusgs_sweep_kernel<S, BB, 0><<<g, block, 0, s>>>(t0, t1, N, P, var0, nei, fa, rv, J, LU,
-                                                                          rhs, du, sp)));
-    } else if (P == 6) {
-        UCFD_BSW(B, (fs_blusgs_sweep_kernel<S, BB, 6><<<g, block, 0, s>>>(t0, t1, N, P, var0, nei, fa, rv, J, LU,
-                                                                          rhs, du, sp)));
-    } else if (P == 4) {
-        UCFD_BSW(B, (fs_blusgs_sweep_kernel<S, BB, 4><<<g, block, 0, s>>>(t0, t1, N, P, var0, nei, fa, rv, J, LU,
-                                                                          rhs, du, sp)));
-    } else {
-        UCFD_BSW(B, (fs_blusgs_sweep_kernel<S, BB, 0><<<g, block, 0, s>>>(t0, t1, N, P, var0, nei, fa, rv, J, LU,
-                                                                          rhs, du, sp)));
+    if (variant != 1 && (P == 6 || P == 4)) {
+        if constexpr (std::is_same<S, float>::value) {
+            if (kFold && B == 5 && t1 - t0 <= kSmallLevel) {
+                if (P == 6) sweep_small_go<5, 6>(s, t0, t1, N, var0, nei, J, rhs, du, sp);
+                else sweep_small_go<5, 4>(s, t0, t1, N, var0, nei, J, rhs, du, sp);
+                return;
+            }
+        }
+        if (P == 6) {
+            UCFD_BSW(B, (sweep_dep_go<S, BB, 6>(g, block, s, t0, t1, N, P, var0, nei, fa, rv, J, LU, rhs, du, sp)));
+        } else {
+            UCFD_BSW(B, (sweep_dep_go<S, BB, 4>(g, block, s, t0, t1, N, P, var0, nei, fa, rv, J, LU, rhs, du, sp)));
+        }
+        return;
     }
+    UCFD_BSW(B, (fs_blusgs_sweep_kernel<S, BB, 0><<<g, block, 0, s>>>(t0, t1, N, P, var0, nei, fa, rv, J, LU, rhs, du,
+                                                                      sp)));
 }
 
 template <typename S>
