@@ -368,6 +368,10 @@ void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent =
     a.nei = s->d_nei.p;
     a.fa = geo_fa<S>(s);
     a.rv = geo_rv<S>(s);
+    if constexpr (std::is_same<S, double>::value) {
+        a.fa = s->fv64.p;  // face area * rcp_vol
+        a.rv = nullptr;
+    }
     a.nrm = w.nrm.p;
     a.lam = rans ? w.lamT.p : w.lamN.p;
     a.tlam = sys == 2 ? w.lamT.p : nullptr;

@@ -76,7 +76,8 @@ __device__ __forceinline__ void ludcmp_dev(T *A) {
     }
 }
 
-// lusub: src/lusgs/inverse.h:51-80 (unit-lower forward, upper backward).
+// lusub: src/lusgs/inverse.h:51-80 (unit-lower forward, upper backward; the
+// sums start from their first product instead of 0 + it).
 // RCP: the diagonal holds reciprocal pivots (ludcmp_dev RSTORE): multiply.
 // (B == 1 stores the reciprocal in both forms, inverse.h:16.)
 template <typename T, int B, bool RCP = false>
@@ -86,18 +87,18 @@ __device__ __forceinline__ void lusub_dev(const T *LU, T *b) {
     } else {
 #pragma unroll
         for (int row = 1; row < B; ++row) {
-            T v = T(0);
+            T v = LU[row * B] * b[0];
 #pragma unroll
-            for (int col = 0; col < row; ++col) v += LU[row * B + col] * b[col];
+            for (int col = 1; col < row; ++col) v += LU[row * B + col] * b[col];
             b[row] -= v;
         }
         if constexpr (RCP) b[B - 1] *= LU[B * B - 1];
         else b[B - 1] /= LU[B * B - 1];
 #pragma unroll
         for (int row = B - 2; row > -1; --row) {
-            T v = T(0);
+            T v = LU[row * B + row + 1] * b[row + 1];
 #pragma unroll
-            for (int col = row + 1; col < B; ++col) v += LU[row * B + col] * b[col];
+            for (int col = row + 2; col < B; ++col) v += LU[row * B + col] * b[col];
             if constexpr (RCP) b[row] = (b[row] - v) * LU[row * B + row];
             else b[row] = (b[row] - v) / LU[row * B + row];
         }

@@ -31,7 +31,11 @@ __device__ __forceinline__ T ld_once(const T *p) {
 // row reads at its neighbours, stays in L2 (the matvec; the preconditioner
 // sweeps keep cached loads, which measured faster there: the last colour of
 // the lower sweep is the first of the upper one).
-template <typename Tv, typename Tx, typename Ta, int B, int PW, int SGN, bool CS = false>
+// ZERO: acc starts as all zeros (the first block's sums are stored, not
+// added).  A block row's sum starts from its first product (the reference's
+// 0 + x differs from x in the sign of a zero only): with both, the exact
+// FP64 row of five blocks takes 245 FP64 instructions instead of 275.
+template <typename Tv, typename Tx, typename Ta, int B, int PW, int SGN, bool CS = false, bool ZERO = false>
 __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, const int *col, const Tv *val,
                                                  const Tx *x, Ta *acc) {
     constexpr int B2 = B * B;
@@ -54,10 +58,11 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
                 const Tv *vp = val + (long long)p * B2 * bn + k;
 #pragma unroll
                 for (int r = 0; r < B; ++r) {
-                    Ta v = Ta(0);
+                    Ta v = (Ta)ld_once<CS>(vp + (long long)(r * B) * bn) * xv[p][0];
 #pragma unroll
-                    for (int cc = 0; cc < B; ++cc) v += (Ta)ld_once<CS>(vp + (long long)(r * B + cc) * bn) * xv[p][cc];
-                    if (SGN > 0) acc[r] += v;
+                    for (int cc = 1; cc < B; ++cc) v += (Ta)ld_once<CS>(vp + (long long)(r * B + cc) * bn) * xv[p][cc];
+                    if (ZERO && SGN > 0 && p == 0) acc[r] = v;
+                    else if (SGN > 0) acc[r] += v;
                     else acc[r] -= v;
                 }
             }
@@ -72,9 +77,9 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
             const Tv *vp = val + (long long)p * B2 * bn + k;
 #pragma unroll
             for (int r = 0; r < B; ++r) {
-                Ta v = Ta(0);
+                Ta v = (Ta)ld_once<CS>(vp + (long long)(r * B) * bn) * xv[0];
 #pragma unroll
-                for (int cc = 0; cc < B; ++cc) v += (Ta)ld_once<CS>(vp + (long long)(r * B + cc) * bn) * xv[cc];
+                for (int cc = 1; cc < B; ++cc) v += (Ta)ld_once<CS>(vp + (long long)(r * B + cc) * bn) * xv[cc];
                 if (SGN > 0) acc[r] += v;
                 else acc[r] -= v;
             }
@@ -87,20 +92,27 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
 // read (the BLAS convention): the reference forms beta*y regardless, which
 // turns an uninitialised y holding NaN or Inf into NaN; for a finite y the
 // results agree (up to the sign of a zero).
+// form (from alpha and beta, picked on the host): 1 y = A x, 2 y -= A x,
+// 3 y = alpha A x, 0 the general form; 1 and 2 give the values of the general
+// form with alpha = 1, beta = 0 and alpha = -1, beta = 1 without its products
+// and, in FP64, without a comparison per row on the FP64 pipe.
 template <typename Tv, typename Ta, int B, int PW>
 __global__ void __launch_bounds__(256) bsr_spmv_kernel(int bn, int P, const int *col, const Tv *val,
                                                        double alpha, const double *x, double beta,
-                                                       double *y) {
+                                                       double *y, int form) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= bn) return;
     Ta acc[B];
 #pragma unroll
     for (int r = 0; r < B; ++r) acc[r] = Ta(0);
-    ell_row_products<Tv, double, Ta, B, PW, +1, true>(i, bn, P, col, val, x, acc);
+    ell_row_products<Tv, double, Ta, B, PW, +1, true, true>(i, bn, P, col, val, x, acc);
 #pragma unroll
     for (int r = 0; r < B; ++r) {
         const long long o = (long long)i * B + r;
-        y[o] = beta == 0.0 ? alpha * (double)acc[r] : alpha * (double)acc[r] + beta * y[o];
+        if (form == 1) y[o] = (double)acc[r];
+        else if (form == 2) y[o] = y[o] - (double)acc[r];
+        else if (form == 3) y[o] = alpha * (double)acc[r];
+        else y[o] = alpha * (double)acc[r] + beta * y[o];
     }
 }
 
@@ -209,7 +221,7 @@ __global__ void __launch_bounds__(256) pc_upper_kernel(int t0, int t1, int bn, i
     if constexpr (MODE == PC_BLUSGS) {
 #pragma unroll
         for (int r = 0; r < B; ++r) arr[r] = T(0);
-        ell_row_products<T, T, T, B, PW, +1>(k, bn, PU, Ucol, Uval, b, arr);
+        ell_row_products<T, T, T, B, PW, +1, false, true>(k, bn, PU, Ucol, Uval, b, arr);
     } else {
 #pragma unroll
         for (int r = 0; r < B; ++r) arr[r] = b[(long long)k * B + r];

@@ -43,6 +43,26 @@ __device__ __forceinline__ T add_prod(T acc, T a, T b) {
     else return acc + a * b;
 }
 
+// x / 2 and p < floor on the integer pipe where the operands are ordinary
+// numbers: an FP64 multiplication or comparison occupies a SM sub-partition's
+// FP64 pipe for 64 clocks, a few integer instructions for 3.  half lowers the
+// exponent by one where the result stays normal; below answers no where x is
+// positive with a larger high word than the floor (all other cases, NaN and
+// negative values among them, compare as usual).
+__device__ __forceinline__ float half(float x) { return 0.5f * x; }
+__device__ __forceinline__ double half(double x) {
+    const int hi = __double2hiint(x);
+    if ((unsigned)(hi & 0x7ff00000) - 0x00200000u < 0x7fd00000u)
+        return __hiloint2double(hi - 0x00100000, __double2loint(x));
+    return 0.5 * x;
+}
+__device__ __forceinline__ bool below(float x, float floor) { return x < floor; }
+__device__ __forceinline__ bool below(double x, double floor) {
+    const int hi = __double2hiint(x);
+    if (hi >= 0 && hi > __double2hiint(floor)) return false;
+    return x < floor;
+}
+
 // ns_flux_container: flux.c:29-67.  The pressure floor rewrites the energy
 // of the local copy u (flux.c:51-56), exactly as the reference does.  In
 // FP32 the two divisions by rho are products with one reciprocal.
@@ -50,9 +70,11 @@ template <typename T, int NFV, int NDIMS>
 __device__ __forceinline__ void ns_flux(T gamma, T pmin, T *u, const T *nf, T *f) {
     T rho = u[0];
     T et = u[NFV - 1];
-    T temp = T(0), contrav = T(0);
+    // (the reference's sums start from 0 + x, which differs from x in the
+    // sign of a zero only)
+    T temp = mul_rn(u[1], u[1]), contrav = mul_rn(u[1], nf[0]);
 #pragma unroll
-    for (int i = 0; i < NDIMS; ++i) {
+    for (int i = 1; i < NDIMS; ++i) {
         contrav = add_prod(contrav, u[i + 1], nf[i]);
         temp = add_prod(temp, u[i + 1], u[i + 1]);
     }
@@ -63,10 +85,10 @@ __device__ __forceinline__ void ns_flux(T gamma, T pmin, T *u, const T *nf, T *f
         ke = T(0.5) * temp * irho;
     } else {
         contrav /= rho;
-        ke = T(0.5) * temp / rho;
+        ke = half(temp) / rho;
     }
     T p = mul_rn(gamma - T(1), et - ke);
-    if (p < pmin) {
+    if (below(p, pmin)) {
         p = pmin;
         et = p / (gamma - T(1)) + ke;
         u[NFV - 1] = et;
@@ -82,9 +104,9 @@ __device__ __forceinline__ void ns_flux(T gamma, T pmin, T *u, const T *nf, T *f
 template <typename T, int NFV, int NDIMS, int NT>
 __device__ __forceinline__ void rans_flux(const T *u, const T *nf, T *f) {
     T rho = u[0];
-    T contrav = T(0);
+    T contrav = mul_rn(u[1], nf[0]);
 #pragma unroll
-    for (int i = 0; i < NDIMS; ++i) contrav = add_prod(contrav, u[i + 1], nf[i]);
+    for (int i = 1; i < NDIMS; ++i) contrav = add_prod(contrav, u[i + 1], nf[i]);
     contrav = div_sweep(contrav, rho);
 #pragma unroll
     for (int i = 0; i < NT; ++i) f[i] = mul_rn(u[NFV + i], contrav);
@@ -279,13 +301,11 @@ __device__ __forceinline__ void face_term(const ScalarSweepArgs<T> &a, T *u, con
         }
     } else {
         T du[NV], f0v[DNV], f1v[DNV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) du[v] = T(0);
-#pragma unroll
-        for (int j = 0; j < DNV; ++j) du[j + NV0] = dn[j];
         // diff_flux: lusgs.c:143-155 (du += u before either flux)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) du[v] += u[v];
+        for (int v = 0; v < NV; ++v) du[v] = u[v];
+#pragma unroll
+        for (int j = 0; j < DNV; ++j) du[j + NV0] = dn[j] + u[j + NV0];
         if constexpr (RANS) {
             rans_flux<T, NFV, NDIMS, NV - NFV>(u, nf, f0v);
             rans_flux<T, NFV, NDIMS, NV - NFV>(du, nf, f1v);
@@ -385,7 +405,8 @@ __device__ __forceinline__ bool no_active_face(const ScalarSweepArgs<T> &a, int 
 // The cell's new increment from its own input, diagonal and df.
 template <typename T>
 __device__ __forceinline__ T sweep_result(bool upper, T own, T df, T dg) {
-    return !upper ? div_sweep(own - T(0.5) * df, dg) : own - div_sweep(T(0.5) * df, dg);
+    const T hd = half(df);
+    return !upper ? div_sweep(own - hd, dg) : own - div_sweep(hd, dg);
 }
 
 template <typename T, int NV, int NFV, int NDIMS, bool RANS, bool COHERENT>
@@ -406,10 +427,11 @@ __device__ __forceinline__ void scalar_sweep_cell(const ScalarSweepArgs<T> &a, i
     }
     const T rvi = a.rv ? __ldg(a.rv + i) : T(1);
 
-    // Active faces three at a time (about 80 registers: occupancy for the
-    // gathers' latency); the terms are added to df in the reference's face
-    // order.
-    constexpr int FB = 3;
+    // Active faces three at a time in FP32 (about 80 registers: occupancy for
+    // the gathers' latency), one at a time in FP64, where three took 188
+    // registers (10 warps per SM) and left the FP64 pipe idle a third of the
+    // time; the terms are added to df in the reference's face order.
+    constexpr int FB = 3, KB = sizeof(T) == 8 ? 1 : FB;
     if (no_active_face(a, lo, hi)) {
     } else if (a.nface <= 2 * FB) {
         // every neighbour index of the cell up front, then its active faces
@@ -417,15 +439,22 @@ __device__ __forceinline__ void scalar_sweep_cell(const ScalarSweepArgs<T> &a, i
 #pragma unroll
         for (int p = 0; p < 2 * FB; ++p) nba[p] = p < a.nface ? __ldg(a.nei + p * ld + i) : -1;
         unsigned m = active_faces<T, 2 * FB>(a, lo, hi, ci, nba);
-        face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, 2 * FB, FB, true>(a, i, rvi, 0, nba, m, nullptr, df);
-        if (m) face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, 2 * FB, FB, true>(a, i, rvi, 0, nba, m, nullptr, df);
+        if constexpr (KB == 1) {
+#pragma unroll 1
+            while (m)
+                face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, 2 * FB, KB, true>(a, i, rvi, 0, nba, m, nullptr, df);
+        } else {
+            face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, 2 * FB, KB, true>(a, i, rvi, 0, nba, m, nullptr, df);
+            if (m) face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, 2 * FB, KB, true>(a, i, rvi, 0, nba, m, nullptr, df);
+        }
     } else {
         for (int f0 = 0; f0 < a.nface; f0 += FB) {
             int nb[FB];
 #pragma unroll
             for (int q = 0; q < FB; ++q) nb[q] = (f0 + q < a.nface) ? __ldg(a.nei + (f0 + q) * ld + i) : -1;
             unsigned m = active_faces<T, FB>(a, lo, hi, ci, nb);
-            face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, FB, FB, true>(a, i, rvi, f0, nb, m, nullptr, df);
+#pragma unroll 1
+            while (m) face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, FB, KB, true>(a, i, rvi, f0, nb, m, nullptr, df);
         }
     }
 #pragma unroll
@@ -525,8 +554,13 @@ __device__ __forceinline__ void scalar_sweep_cell_both(const ScalarSweepArgs<T> 
 #pragma unroll
         for (int p = 0; p < 2 * FB; ++p) nba[p] = p < a.nface ? __ldg(a.nei + p * ld + i) : -1;
         unsigned m = active_faces<T, 2 * FB>(a, lo, hi, ci, nba);
-        face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, FB>(a, i, rvi, 0, nba, m, df);
-        if (m) face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, FB>(a, i, rvi, 0, nba, m, df);
+        if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+            while (m) face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, 1>(a, i, rvi, 0, nba, m, df);
+        } else {
+            face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, FB>(a, i, rvi, 0, nba, m, df);
+            if (m) face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, FB>(a, i, rvi, 0, nba, m, df);
+        }
     } else {
         for (int f0 = 0; f0 < a.nface; f0 += FB) {
             int nb[FB];
@@ -559,12 +593,13 @@ __device__ __forceinline__ void ns_flux_lane(double gamma, double pmin, const do
     double dot = mul_rn(u[1], h ? u[1] : n[0]);
 #pragma unroll
     for (int d = 1; d < NDIMS; ++d) dot = add_prod(dot, u[d + 1], h ? u[d + 1] : n[d]);
-    const double q = mul_rn(h ? 0.5 : 1.0, dot) / u[0];  // lane 0: m.n / rho; lane 1: 0.5 m.m / rho
+    const double hd = half(dot);
+    const double q = (h ? hd : dot) / u[0];  // lane 0: m.n / rho; lane 1: 0.5 m.m / rho
     const double o = __shfl_xor_sync(0xffffffffu, q, 1);
     const double c = h ? o : q, ke = h ? q : o;
     double et = u[NFV - 1];
     double p = mul_rn(gamma - 1.0, et - ke);
-    if (p < pmin) {
+    if (below(p, pmin)) {
         p = pmin;
         et = p / (gamma - 1.0) + ke;
     }

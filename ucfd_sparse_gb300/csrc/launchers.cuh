@@ -571,16 +571,17 @@ void bsr_spmv(int B, int bn, int P, const int *col, const Tv *val, double alpha,
     if (bn <= 0) return;
     block = spread_block<Ta>(bn, block);
     const unsigned g = grid_for(bn, block);
+    const int form = beta == 0.0 ? (alpha == 1.0 ? 1 : 3) : beta == 1.0 && alpha == -1.0 ? 2 : 0;
     // unrolled rows for the 5x5 systems (tets: diag + 4 faces; hexes: + 6)
     if (B == 5 && P <= 5) {
-        bsr_spmv_kernel<Tv, Ta, 5, 5><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y);
+        bsr_spmv_kernel<Tv, Ta, 5, 5><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form);
         return;
     }
     if (B == 5 && P <= 7) {
-        bsr_spmv_kernel<Tv, Ta, 5, 7><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y);
+        bsr_spmv_kernel<Tv, Ta, 5, 7><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form);
         return;
     }
-    UCFD_KSW(B, (bsr_spmv_kernel<Tv, Ta, BB, 0><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y)));
+    UCFD_KSW(B, (bsr_spmv_kernel<Tv, Ta, BB, 0><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form)));
 }
 
 template <typename Tl>
