@@ -69,7 +69,8 @@ void adjoint(int neles, int nface, int nvars, int nfvars, int ndims, const int *
     for (int c = 0; c < ncolors; ++c) {
         a.t0 = c == 0 ? 0 : ranges[c - 1];
         a.t1 = ranges[c];
-        kfast::adj_upper<T>(a, nfvars, ndims, g, pm, fnv, vec, fspr, upts, diag, dub, dq, gdq, qbar, dbar, gfspr, s);
+        kfast::adj_upper<T>(a, nfvars, ndims, g, pm, fnv, vec, fspr, upts, diag, dub, dq, gdq, qbar, wbuf, dbar,
+                            gfspr, s);
     }
     for (int c = ncolors - 1; c >= 0; --c) {
         a.t0 = c == 0 ? 0 : ranges[c - 1];

@@ -52,7 +52,7 @@ UCFD_INST_T(float)
 #undef UCFD_INST_T
 #define UCFD_INST_ADJ(T)                                                                                       \
     template void adj_upper<T>(const ::ucfd::AdjArgs &, int, int, T, T, const T *, const T *, const T *,      \
-                               const T *, const T *, const T *, const T *, const T *, T *, T *, T *,          \
+                               const T *, const T *, const T *, const T *, const T *, T *, T *, T *, T *,     \
                                cudaStream_t);                                                                 \
     template void adj_lower<T>(const ::ucfd::AdjArgs &, int, int, T, T, T, const T *, const T *, const T *,    \
                                const T *, const T *, const T *, const T *, const T *, T *, const T *, T *,    \

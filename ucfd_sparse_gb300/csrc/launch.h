@@ -127,7 +127,7 @@
     template <typename T>                                                                          \
     void adj_upper(const ::ucfd::AdjArgs &a, int nfv, int ndims, T gamma, T pmin, const T *fnv,    \
                    const T *vec, const T *fspr, const T *upts, const T *diag, const T *dub,        \
-                   const T *dq, const T *gdq, T *qbar, T *dbar, T *gfspr, cudaStream_t s);         \
+                   const T *dq, const T *gdq, T *qbar, T *wbuf, T *dbar, T *gfspr, cudaStream_t s);         \
     template <typename T>                                                                          \
     void adj_lower(const ::ucfd::AdjArgs &a, int nfv, int ndims, T gamma, T pmin, T factor,        \
                    const T *fnv, const T *vec, const T *fspr, const T *dt, const T *upts,          \

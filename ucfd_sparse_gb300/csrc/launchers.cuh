@@ -14,19 +14,18 @@ namespace UCFD_KNS {
 // ---- adjoint of the colored LU-SGS step --------------------------------------
 template <typename T>
 void adj_upper(const ::ucfd::AdjArgs &a, int nfv, int ndims, T gamma, T pmin, const T *fnv, const T *vec,
-               const T *fspr, const T *upts, const T *diag, const T *dub, const T *dq, const T *gdq, T *qbar, T *dbar,
-               T *gfspr, cudaStream_t s) {
+               const T *fspr, const T *upts, const T *diag, const T *dub, const T *dq, const T *gdq, T *qbar, T *wbuf,
+               T *dbar, T *gfspr, cudaStream_t s) {
     const int n = a.t1 - a.t0;
     if (n <= 0) return;
     const int block = spread_block<T>(n, 0);
     if (nfv == 5 && ndims == 3)
-        adj_upper_kernel<T, 5, 5, 3><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag, dub,
-                                                                     dq, gdq, qbar, dbar, gfspr);
-    else if (nfv == 4 && ndims == 2)
-        adj_upper_kernel<T, 4, 4, 2><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag, dub,
-                                                                     dq, gdq, qbar, dbar, gfspr);
-    else
-        ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "adjoint built for nfvars/ndims 5/3 and 4/2 only");
+        return adj_upper_kernel<T, 5, 3><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag,
+                                                                              dub, dq, gdq, qbar, wbuf, dbar, gfspr);
+    if (nfv == 4 && ndims == 2)
+        return adj_upper_kernel<T, 4, 2><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, fnv, vec, fspr, upts, diag,
+                                                                              dub, dq, gdq, qbar, wbuf, dbar, gfspr);
+    ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "adjoint built for nfvars/ndims 5/3 and 4/2 only");
 }
 
 template <typename T>
@@ -37,13 +36,12 @@ void adj_lower(const ::ucfd::AdjArgs &a, int nfv, int ndims, T gamma, T pmin, T 
     if (n <= 0) return;
     const int block = spread_block<T>(n, 0);
     if (nfv == 5 && ndims == 3)
-        adj_lower_kernel<T, 5, 5, 3><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, factor, fnv, vec, fspr, dt, upts,
-                                                                     diag, dub, qbar, wbuf, dbar, grhs, gdt, gfspr);
-    else if (nfv == 4 && ndims == 2)
-        adj_lower_kernel<T, 4, 4, 2><<<grid_for(n, block), block, 0, s>>>(a, gamma, pmin, factor, fnv, vec, fspr, dt, upts,
-                                                                     diag, dub, qbar, wbuf, dbar, grhs, gdt, gfspr);
-    else
-        ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "adjoint built for nfvars/ndims 5/3 and 4/2 only");
+        return adj_lower_kernel<T, 5, 3><<<grid_for(n, block), block, 0, s>>>(
+            a, gamma, pmin, factor, fnv, vec, fspr, dt, upts, diag, dub, qbar, wbuf, dbar, grhs, gdt, gfspr);
+    if (nfv == 4 && ndims == 2)
+        return adj_lower_kernel<T, 4, 2><<<grid_for(n, block), block, 0, s>>>(
+            a, gamma, pmin, factor, fnv, vec, fspr, dt, upts, diag, dub, qbar, wbuf, dbar, grhs, gdt, gfspr);
+    ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "adjoint built for nfvars/ndims 5/3 and 4/2 only");
 }
 
 // ---- scalar LU-SGS ---------------------------------------------------------
