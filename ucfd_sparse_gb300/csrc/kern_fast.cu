@@ -43,10 +43,11 @@ namespace kfast {
                                  double *, int, cudaStream_t);                                                 \
     template void pc_prepare<T>(int, int, const int *, const long long *, const double *, double *, T *, int,  \
                                 cudaStream_t);                                                                 \
-    template void pc_lower<T>(int, int, int, int, int, const int *, const T *, const T *, T *, int, int,       \
-                              cudaStream_t);                                                                   \
-    template void pc_upper<T>(int, int, int, int, int, const int *, const T *, const T *, T *, int, int,       \
-                              cudaStream_t);
+    template int pc_stride<T>(int);                                                                            \
+    template void pc_lower<T>(int, int, int, int, int, const int *, const T *, const T *, const int *,         \
+                              double *, T *, int, int, cudaStream_t);                                          \
+    template void pc_upper<T>(int, int, int, int, int, const int *, const T *, const T *, const int *,         \
+                              double *, T *, int, int, cudaStream_t);
 UCFD_INST_T(double)
 UCFD_INST_T(float)
 #undef UCFD_INST_T
@@ -63,12 +64,6 @@ UCFD_INST_ADJ(float)
 template void fs_blusgs_residual<double, float>(int, long long, int, int, int, const int *, const double *,
                                                 const double *, const double *, const double *, const double *,
                                                 const double *, float *, double *, int, int *, cudaStream_t);
-template void gather_rows<double, double>(int, int, const int *, const double *, double *, cudaStream_t);
-template void scatter_rows<double, double>(int, int, const int *, const double *, double *, cudaStream_t);
-template void gather_rows<double, float>(int, int, const int *, const double *, float *, cudaStream_t);
-template void scatter_rows<float, double>(int, int, const int *, const float *, double *, cudaStream_t);
-template void ell_gather<double>(int, int, int, const int *, const double *, double *, cudaStream_t);
-template void ell_gather<float>(int, int, int, const int *, const double *, float *, cudaStream_t);
 template void convert<double, float>(long long, const double *, float *, cudaStream_t);
 template void convert<float, double>(long long, const float *, double *, cudaStream_t);
 template void axpy_into<float>(long long, const float *, double *, cudaStream_t);

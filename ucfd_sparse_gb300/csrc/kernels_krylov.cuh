@@ -20,6 +20,40 @@ __device__ __forceinline__ T ld_once(const T *p) {
     else return __ldg(p);
 }
 
+// Row g of a gathered vector, XS entries per row, the first B used.  The
+// lanes of a warp gather from different lines, so each load instruction
+// costs the L1 one pass per lane whatever its width: a row is read with the
+// fewest loads its alignment allows.
+//   FP64, B = XS = 5, VEC (base 16-byte aligned): two 16-byte loads and one
+//     8-byte load, the odd entry first in odd rows (the FP32 matvec, 5.3M
+//     rows: 711 -> 586 us with the conversions below; the FP64 kernels, bound
+//     by the FP64 pipe, gain nothing from it and do not use it);
+//   FP32, XS = 8: one 16-byte load and one per entry above 4;
+//   else one load per entry.
+template <typename Tx, int B, int XS, bool VEC>
+__device__ __forceinline__ void load_row(const Tx *x, long long g, Tx *v) {
+    const Tx *q = x + g * XS;
+    if constexpr (VEC && B == 5 && XS == 5 && sizeof(Tx) == 8) {
+        const int odd = (int)(g & 1);
+        const double2 a = *reinterpret_cast<const double2 *>(q + odd);
+        const double2 b = *reinterpret_cast<const double2 *>(q + odd + 2);
+        const double o = q[odd ? 0 : 4];
+        v[0] = odd ? o : a.x;
+        v[1] = odd ? a.x : a.y;
+        v[2] = odd ? a.y : b.x;
+        v[3] = odd ? b.x : b.y;
+        v[4] = odd ? b.y : o;
+    } else if constexpr (XS == 8 && B >= 4 && sizeof(Tx) == 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(q);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+#pragma unroll
+        for (int c = 4; c < B; ++c) v[c] = q[c];
+    } else {
+#pragma unroll
+        for (int c = 0; c < B; ++c) v[c] = q[c];
+    }
+}
+
 // acc[r] += SGN * sum over the ELL row k of (block_p x_{col_p})[r], entries in
 // stored order, each block product summed over its columns first (the
 // reference's order, sparsemat.c:82-97, blusgs.c:113-124).  PW > 0: the
@@ -35,7 +69,8 @@ __device__ __forceinline__ T ld_once(const T *p) {
 // added).  A block row's sum starts from its first product (the reference's
 // 0 + x differs from x in the sign of a zero only): with both, the exact
 // FP64 row of five blocks takes 245 FP64 instructions instead of 275.
-template <typename Tv, typename Tx, typename Ta, int B, int PW, int SGN, bool CS = false, bool ZERO = false>
+// x holds XS entries per row (load_row).
+template <typename Tv, typename Tx, typename Ta, int B, int PW, int SGN, bool CS, bool ZERO, int XS, bool VEC>
 __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, const int *col, const Tv *val,
                                                  const Tx *x, Ta *acc) {
     constexpr int B2 = B * B;
@@ -47,8 +82,10 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
 #pragma unroll
         for (int p = 0; p < PW; ++p) {
             const long long g = c[p] >= 0 ? c[p] : 0;  // padding: any valid address
+            Tx xr[B];
+            load_row<Tx, B, XS, VEC>(x, g, xr);
 #pragma unroll
-            for (int cc = 0; cc < B; ++cc) xv[p][cc] = (Ta)x[g * B + cc];
+            for (int cc = 0; cc < B; ++cc) xv[p][cc] = convert_to<Ta>(xr[cc]);
         }
         bool live = true;
 #pragma unroll
@@ -71,9 +108,11 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
         for (int p = 0; p < P; ++p) {
             const int c = ld_once<CS>(col + (long long)p * bn + k);
             if (c < 0) break;
+            Tx xr[B];
+            load_row<Tx, B, XS, VEC>(x, c, xr);
             Ta xv[B];
 #pragma unroll
-            for (int cc = 0; cc < B; ++cc) xv[cc] = (Ta)x[(long long)c * B + cc];
+            for (int cc = 0; cc < B; ++cc) xv[cc] = convert_to<Ta>(xr[cc]);
             const Tv *vp = val + (long long)p * B2 * bn + k;
 #pragma unroll
             for (int r = 0; r < B; ++r) {
@@ -96,7 +135,8 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
 // 3 y = alpha A x, 0 the general form; 1 and 2 give the values of the general
 // form with alpha = 1, beta = 0 and alpha = -1, beta = 1 without its products
 // and, in FP64, without a comparison per row on the FP64 pipe.
-template <typename Tv, typename Ta, int B, int PW>
+// VEC: x and y 16-byte aligned.
+template <typename Tv, typename Ta, int B, int PW, bool VEC>
 __global__ void __launch_bounds__(256) bsr_spmv_kernel(int bn, int P, const int *col, const Tv *val,
                                                        double alpha, const double *x, double beta,
                                                        double *y, int form) {
@@ -105,43 +145,59 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int bn, int P, const int 
     Ta acc[B];
 #pragma unroll
     for (int r = 0; r < B; ++r) acc[r] = Ta(0);
-    ell_row_products<Tv, double, Ta, B, PW, +1, true, true>(i, bn, P, col, val, x, acc);
+    ell_row_products<Tv, double, Ta, B, PW, +1, true, true, B, VEC>(i, bn, P, col, val, x, acc);
 #pragma unroll
     for (int r = 0; r < B; ++r) {
         const long long o = (long long)i * B + r;
-        if (form == 1) y[o] = (double)acc[r];
-        else if (form == 2) y[o] = y[o] - (double)acc[r];
-        else if (form == 3) y[o] = alpha * (double)acc[r];
-        else y[o] = alpha * (double)acc[r] + beta * y[o];
+        if (form == 1) y[o] = to_double(acc[r]);
+        else if (form == 2) y[o] = y[o] - to_double(acc[r]);
+        else if (form == 3) y[o] = alpha * to_double(acc[r]);
+        else y[o] = alpha * to_double(acc[r]) + beta * y[o];
     }
 }
 
 // Values of a CSR-of-blocks array (row-major B x B blocks in slot order)
 // into the ELL-of-blocks layout: ELL entry (p, k) takes the block at slot
-// src[p*bn + k] (src < 0: padding, zeros).  One thread per ELL entry: the
-// writes coalesce over k, and a thread's B*B reads are one contiguous block
-// requested all at once.  T = float rounds the FP64 values.
-template <typename T, int B>
-__global__ void __launch_bounds__(256) ell_gather_kernel(int bn, int P, const int *src, const double *vals,
-                                                         T *out) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)P * bn) return;
-    constexpr int B2 = B * B;
-    const int p = (int)(t / bn);
-    const int k = (int)(t - (long long)p * bn);
-    const int q = __ldg(src + t);
-    T *o = out + (long long)p * B2 * bn + k;
-    double v[B2];
-    if (q >= 0) {
-        const double *blk = vals + (long long)q * B2;
+// src[p*bn + k] (src < 0: padding, zeros), into out64 and / or out32 (rounded
+// to FP32) -- one pass for both, since reading the values is half of its
+// traffic.  A warp takes 32 consecutive rows of one p: it reads the blocks
+// one after the other, its lanes along a block (whole sectors instead of one
+// 8-byte word of every row's block per load), into shared memory, then each
+// lane writes its row's values, coalesced over the rows.  Bound by HBM: 5.3M
+// tetrahedral rows, FP64 and FP32 copies 3.77 -> 2.2 ms (two passes, a lane
+// per block, conversions on the FP64 pipe).
+template <int B>
+constexpr int kGatherWarps = B > 6 ? 2 : 4;  // tiles of at most 48 KB per block
+template <int B>
+__global__ void __launch_bounds__(32 * kGatherWarps<B>) ell_gather_kernel(int bn, int P, const int *src, const double *vals,
+                                                         double *out64, float *out32) {
+    constexpr int B2 = B * B, LD = B2 | 1;  // odd row stride: lanes reading one entry of 32 rows use all banks
+    constexpr int W = kGatherWarps<B>;
+    __shared__ double sm[W][32 * LD];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int groups = (bn + 31) >> 5;
+    const long long w = (long long)blockIdx.x * W + wid;
+    if (w >= (long long)P * groups) return;
+    const int p = (int)(w % P);  // the P entries of 32 rows next to each other: whole rows are read at a time
+    const int k = ((int)(w / P) << 5) + lane;
+    const int q = k < bn ? __ldg(src + (long long)p * bn + k) : -1;
+    double *t = sm[wid];
+    // entries lane, lane + 32, ... of the 32 blocks, all loads in flight
 #pragma unroll
-        for (int e = 0; e < B2; ++e) v[e] = __ldg(blk + e);
-    } else {
-#pragma unroll
-        for (int e = 0; e < B2; ++e) v[e] = 0.0;
+    for (int i = 0; i < B2; ++i) {
+        const int e = i * 32 + lane, r = e / B2, j = e - r * B2;
+        const int qr = __shfl_sync(0xffffffffu, q, r);
+        t[r * LD + j] = qr >= 0 ? __ldg(vals + (long long)qr * B2 + j) : 0.0;
     }
+    __syncwarp();
+    if (k >= bn) return;
+    const long long o = (long long)p * B2 * bn + k;
 #pragma unroll
-    for (int e = 0; e < B2; ++e) o[(long long)e * bn] = (T)v[e];
+    for (int e = 0; e < B2; ++e) {
+        const double v = t[lane * LD + e];
+        if (out64) out64[o + (long long)e * bn] = v;
+        if (out32) out32[o + (long long)e * bn] = to_float(v);
+    }
 }
 
 // Order-independent 64-bit fingerprint of an int array: out += sum over i
@@ -176,8 +232,8 @@ __global__ void pc_prepare_kernel(int bn, const int *perm, const long long *dslo
     if (factor) ludcmp_dev<double, B, kFold, kFold>(d);
 #pragma unroll
     for (int e = 0; e < B2; ++e) {
-        LU64[(long long)e * bn + k] = d[e];
-        if (LU_l) LU_l[(long long)e * bn + k] = (Tl)d[e];
+        if (LU64) LU64[(long long)e * bn + k] = d[e];
+        if (LU_l) LU_l[(long long)e * bn + k] = convert_to<Tl>(d[e]);
     }
 }
 
@@ -191,41 +247,61 @@ __global__ void pc_prepare_kernel(int bn, const int *perm, const long long *dslo
 //     kept diagonal a_ii (LU holds a_ii, not its reciprocal).
 enum { PC_BLUSGS = 0, PC_BILU = 1, PC_ILU = 2 };
 
-template <typename T, int B, int PW, int MODE>
+// Both kernels also carry the vector between the caller's order and the
+// level-major order (and FP64 and FP32), which two passes of their own did
+// before: a row of the lower sweep starts from row perm[k] of the caller's b,
+// and the upper sweep stores its result there as well.  x, the working
+// vector, has XS entries per row (8 in FP32: a gathered row is one 32-byte
+// sector).  Without a permutation in FP64, x is b itself.
+template <typename T, int B, int XS>
+__device__ __forceinline__ void store_row(T *x, long long k, const T *v) {
+    T *q = x + k * XS;
+    if constexpr (XS == 8 && B >= 4 && sizeof(T) == 4) {
+        *reinterpret_cast<float4 *>(q) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+        for (int c = 4; c < B; ++c) q[c] = v[c];
+    } else {
+#pragma unroll
+        for (int c = 0; c < B; ++c) q[c] = v[c];
+    }
+}
+
+template <typename T, int B, int PW, int MODE, int XS>
 __global__ void __launch_bounds__(256) pc_lower_kernel(int t0, int t1, int bn, int PL, const int *Lcol,
-                                                       const T *Lval, const T *LU, T *b) {
+                                                       const T *Lval, const T *LU, const int *perm,
+                                                       const double *b, T *x) {
     const int k = t0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= t1) return;
     constexpr int B2 = B * B;
+    const long long s = perm ? __ldg(perm + k) : k;
     T arr[B];
 #pragma unroll
-    for (int r = 0; r < B; ++r) arr[r] = b[(long long)k * B + r];
-    ell_row_products<T, T, T, B, PW, -1>(k, bn, PL, Lcol, Lval, b, arr);
+    for (int r = 0; r < B; ++r) arr[r] = convert_to<T>(b[s * B + r]);
+    ell_row_products<T, T, T, B, PW, -1, false, false, XS, false>(k, bn, PL, Lcol, Lval, x, arr);
     if constexpr (MODE == PC_BLUSGS) {
         T lu[B2];
 #pragma unroll
         for (int e = 0; e < B2; ++e) lu[e] = __ldg(LU + (long long)e * bn + k);
         lusub_dev<T, B, kFold>(lu, arr);  // reciprocal pivots in the fast build (pc_prepare)
     }
-#pragma unroll
-    for (int r = 0; r < B; ++r) b[(long long)k * B + r] = arr[r];
+    store_row<T, B, XS>(x, k, arr);
 }
 
-template <typename T, int B, int PW, int MODE>
+template <typename T, int B, int PW, int MODE, int XS>
 __global__ void __launch_bounds__(256) pc_upper_kernel(int t0, int t1, int bn, int PU, const int *Ucol,
-                                                       const T *Uval, const T *LU, T *b) {
+                                                       const T *Uval, const T *LU, const int *perm, double *b,
+                                                       T *x) {
     const int k = t0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= t1) return;
     constexpr int B2 = B * B;
-    T arr[B];
+    T arr[B], own[B];
     if constexpr (MODE == PC_BLUSGS) {
 #pragma unroll
         for (int r = 0; r < B; ++r) arr[r] = T(0);
-        ell_row_products<T, T, T, B, PW, +1, false, true>(k, bn, PU, Ucol, Uval, b, arr);
+        ell_row_products<T, T, T, B, PW, +1, false, true, XS, false>(k, bn, PU, Ucol, Uval, x, arr);
     } else {
-#pragma unroll
-        for (int r = 0; r < B; ++r) arr[r] = b[(long long)k * B + r];
-        ell_row_products<T, T, T, B, PW, -1>(k, bn, PU, Ucol, Uval, b, arr);
+        load_row<T, B, XS, false>(x, k, arr);
+        ell_row_products<T, T, T, B, PW, -1, false, false, XS, false>(k, bn, PU, Ucol, Uval, x, arr);
     }
     if constexpr (MODE == PC_ILU) {
         static_assert(B == 1, "scalar ILU is B = 1");
@@ -239,10 +315,16 @@ __global__ void __launch_bounds__(256) pc_upper_kernel(int t0, int t1, int bn, i
         if constexpr (MODE == PC_BLUSGS) lusub_dev<T, B, kFold>(lu, arr);
         else lusub_dev<T, B>(lu, arr);
     }
+    if constexpr (MODE == PC_BLUSGS) {
+        load_row<T, B, XS, false>(x, k, own);
 #pragma unroll
-    for (int r = 0; r < B; ++r) {
-        if constexpr (MODE == PC_BLUSGS) b[(long long)k * B + r] -= arr[r];
-        else b[(long long)k * B + r] = arr[r];
+        for (int r = 0; r < B; ++r) arr[r] = own[r] - arr[r];
+    }
+    store_row<T, B, XS>(x, k, arr);
+    if ((const void *)x != (const void *)b) {
+        const long long s = perm ? __ldg(perm + k) : k;
+#pragma unroll
+        for (int r = 0; r < B; ++r) b[s * B + r] = to_double(arr[r]);
     }
 }
 
@@ -307,24 +389,100 @@ __global__ void ilu_factor_kernel(int t0, int t1, const int *rows, const int *ro
     }
 }
 
-// Vector permutation / precision change between the caller's order and
-// the level-major order of a preconditioner: dst[k] = src[perm[k]].
-template <typename Ts, typename Td>
-__global__ void gather_rows_kernel(int bn, int B, const int *perm, const Ts *src, Td *dst) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)bn * B) return;
-    const long long k = t / B, r = t - k * B;
-    const long long s = perm ? (long long)perm[k] : k;
-    dst[t] = (Td)src[s * B + r];
-}
-
-template <typename Ts, typename Td>
-__global__ void scatter_rows_kernel(int bn, int B, const int *perm, const Ts *src, Td *dst) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)bn * B) return;
-    const long long k = t / B, r = t - k * B;
-    const long long d = perm ? (long long)perm[k] : k;
-    dst[d * B + r] = (Td)src[t];
+// The block factorisation of one level with B lanes per row (32 / B rows per
+// warp): lane r owns row r of every block of its block row.  A_ik inv(A_kk)
+// and A_ij -= A_ik A_kj are independent in the rows of the block, so a lane
+// issues a fifth of the FP64 instructions that a thread per block row does
+// (they bound it: about 2000 per row in one chain) and touches only entries
+// it wrote itself; the diagonal block's LU passes each finished row from
+// lane to lane.  Same operations on every entry, in the same order.  On
+// 83K rows, exact build: 645 us in three levels with one thread per row.
+template <int B>
+__global__ void __launch_bounds__(32) ilu_factor_rows_kernel(int t0, int t1, const int *rows, const int *rowptr,
+                                                             const int *colidx, const int *diagslots,
+                                                             double *vals) {
+    constexpr int C = 32 / B, B2 = B * B;
+    const int lane = threadIdx.x, c = lane / B, r = lane - c * B, base = c * B;
+    const int t = t0 + blockIdx.x * C + c;
+    const bool valid = c < C && t < t1;
+    double d[B];
+#pragma unroll
+    for (int e = 0; e < B; ++e) d[e] = e == r ? 1.0 : 0.0;
+    long long diag = 0;
+    if (valid) {
+        const int i = rows ? rows[t] : t;
+        const int st = rowptr[i], ed = diagslots[i], jed = rowptr[i + 1];
+        diag = (long long)ed * B2 + r * B;
+        for (int kd = st; kd < ed; ++kd) {
+            const int ck = colidx[kd], kst = rowptr[ck], ked = rowptr[ck + 1];
+            const double *lu = vals + (long long)diagslots[ck] * B2;
+            double *own = vals + (long long)kd * B2 + r * B;
+            double x[B];
+#pragma unroll
+            for (int e = 0; e < B; ++e) x[e] = own[e];
+            // row r of A_ik inv(LU): lusubmattrans_dev
+            x[0] /= lu[0];
+#pragma unroll
+            for (int row = 1; row < B; ++row) {
+                double v = x[0] * lu[row];
+#pragma unroll
+                for (int col = 1; col < row; ++col) v += x[col] * lu[col * B + row];
+                x[row] = (x[row] - v) / lu[row * B + row];
+            }
+#pragma unroll
+            for (int row = B - 2; row > -1; --row) {
+                double v = x[row + 1] * lu[(row + 1) * B + row];
+#pragma unroll
+                for (int col = row + 2; col < B; ++col) v += x[col] * lu[col * B + row];
+                x[row] -= v;
+            }
+#pragma unroll
+            for (int e = 0; e < B; ++e) own[e] = x[e];
+            for (int jj = kd + 1; jj < jed; ++jj) {
+                const int cj = colidx[jj];
+                int iwj = -1;
+                for (int q = kst; q < ked; ++q)
+                    if (colidx[q] == cj) iwj = q;
+                if (iwj < 0) continue;
+                const double *akj = vals + (long long)iwj * B2;
+                double *aij = vals + (long long)jj * B2 + r * B;
+#pragma unroll
+                for (int e = 0; e < B; ++e) {
+                    double v = x[0] * akj[e];
+#pragma unroll
+                    for (int q = 1; q < B; ++q) v += x[q] * akj[q * B + e];
+                    aij[e] -= v;
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < B; ++e) d[e] = vals[diag + e];
+    }
+    __syncwarp();
+    // ludcmp (inverse.h:13-45), row k final at step k
+    double v[B];
+#pragma unroll
+    for (int k = 0; k < B - 1; ++k) {
+        const double piv = __shfl_sync(0xffffffffu, d[k], base + k);
+        double l = 0.0;
+        if (r > k) {
+            l = (k == 0 ? d[0] : d[k] - v[k]) / piv;
+            d[k] = l;
+        }
+#pragma unroll
+        for (int e = k + 1; e < B; ++e) {
+            const double u = __shfl_sync(0xffffffffu, d[e], base + k);
+            if (r > k) v[e] = k == 0 ? l * u : v[e] + l * u;
+        }
+        if (r == k + 1) {
+#pragma unroll
+            for (int e = k + 1; e < B; ++e) d[e] -= v[e];
+        }
+    }
+    if (valid) {
+#pragma unroll
+        for (int e = 0; e < B; ++e) vals[diag + e] = d[e];
+    }
 }
 
 // ---- GMRES(m) device pieces (gmres.c:4-129) --------------------------------

@@ -73,14 +73,7 @@ struct EllBlocks {
     // and/or val32 (rounded to FP32).
     void gather(const double *vals, bool fp64, bool fp32, cudaStream_t s) {
         const size_t n = (size_t)std::max(P, 1) * B * B * bn;
-        if (fp64) {
-            val.ensure(n);
-            kfast::ell_gather<double>(B, bn, P, src.p, vals, val.p, s);
-        }
-        if (fp32) {
-            val32.ensure(n);
-            kfast::ell_gather<float>(B, bn, P, src.p, vals, val32.p, s);
-        }
+        kfast::ell_gather(B, bn, P, src.p, vals, fp64 ? val.ensure(n) : nullptr, fp32 ? val32.ensure(n) : nullptr, s);
     }
 };
 
@@ -325,14 +318,15 @@ struct _Precon {
         }
         L.gather(vd, !fp32, fp32, s);
         U.gather(vd, !fp32, fp32, s);
-        LU64.ensure(B2 * bn);
         const int fac = kind == 0 ? 1 : 0;  // the ILU types arrive factored
         if (fp32) {
-            LU32.ensure(B2 * bn);
-            kfast::pc_prepare<float>(blk, bn, identity ? nullptr : perm.p, dslot.p, vd, LU64.p, LU32.p, fac, s);
+            LU32.ensure(B2 * bn);  // FP32 applies read the rounded factors only
+            kfast::pc_prepare<float>(blk, bn, identity ? nullptr : perm.p, dslot.p, vd, nullptr, LU32.p, fac, s);
         } else if (prec == UCFD_PREC_FP64) {
+            LU64.ensure(B2 * bn);
             kexact::pc_prepare<double>(blk, bn, identity ? nullptr : perm.p, dslot.p, vd, LU64.p, nullptr, fac, s);
         } else {
+            LU64.ensure(B2 * bn);
             kfast::pc_prepare<double>(blk, bn, identity ? nullptr : perm.p, dslot.p, vd, LU64.p, nullptr, fac, s);
         }
         UCFD_CHECK_LAUNCH();
@@ -360,43 +354,30 @@ struct _Precon {
     void apply(double *b, cudaStream_t s) {
         if (none) return;
         UCFD_REQUIRE(prepared, "UCFDPreconPrepare has not been called");
-        const long long n = (long long)bn * blk;
-        const int L_ = sch.nlev;
+        const int *pm = identity ? nullptr : perm.p;
+        const auto levels = [&](auto &&lower, auto &&upper) {
+            for (int l = 0; l < sch.nlev; ++l) lower(sch.lev_off[l], sch.lev_off[l + 1]);
+            for (int l = sch.nlev - 1; l >= 0; --l) upper(sch.lev_off[l], sch.lev_off[l + 1]);
+        };
         if (prec == UCFD_PREC_FP32) {
-            float *x = tmp32.ensure(n);
-            kfast::gather_rows<double, float>(bn, blk, identity ? nullptr : perm.p, b, x, s);
-            for (int l = 0; l < L_; ++l)
-                kfast::pc_lower<float>(blk, sch.lev_off[l], sch.lev_off[l + 1], bn, L.P, L.col.p, L.val32.p, LU32.p, x,
-                                       0, kind, s);
-            for (int l = L_ - 1; l >= 0; --l)
-                kfast::pc_upper<float>(blk, sch.lev_off[l], sch.lev_off[l + 1], bn, U.P, U.col.p, U.val32.p, LU32.p, x,
-                                       0, kind, s);
-            kfast::scatter_rows<float, double>(bn, blk, identity ? nullptr : perm.p, x, b, s);
-        } else {
-            double *x = b;
-            if (!identity) {
-                x = tmp64.ensure(n);
-                kfast::gather_rows<double, double>(bn, blk, perm.p, b, x, s);
-            }
-            const bool ex = prec == UCFD_PREC_FP64;
-            for (int l = 0; l < L_; ++l) {
-                if (ex)
-                    kexact::pc_lower<double>(blk, sch.lev_off[l], sch.lev_off[l + 1], bn, L.P, L.col.p, L.val.p,
-                                             LU64.p, x, 0, kind, s);
-                else
-                    kfast::pc_lower<double>(blk, sch.lev_off[l], sch.lev_off[l + 1], bn, L.P, L.col.p, L.val.p,
-                                            LU64.p, x, 0, kind, s);
-            }
-            for (int l = L_ - 1; l >= 0; --l) {
-                if (ex)
-                    kexact::pc_upper<double>(blk, sch.lev_off[l], sch.lev_off[l + 1], bn, U.P, U.col.p, U.val.p,
-                                             LU64.p, x, 0, kind, s);
-                else
-                    kfast::pc_upper<double>(blk, sch.lev_off[l], sch.lev_off[l + 1], bn, U.P, U.col.p, U.val.p,
-                                            LU64.p, x, 0, kind, s);
-            }
-            if (!identity) kfast::scatter_rows<double, double>(bn, blk, perm.p, x, b, s);
+            float *x = tmp32.ensure((size_t)bn * kfast::pc_stride<float>(blk));
+            levels([&](int a, int z) { kfast::pc_lower<float>(blk, a, z, bn, L.P, L.col.p, L.val32.p, LU32.p, pm, b, x,
+                                                              0, kind, s); },
+                   [&](int a, int z) { kfast::pc_upper<float>(blk, a, z, bn, U.P, U.col.p, U.val32.p, LU32.p, pm, b, x,
+                                                              0, kind, s); });
+            return;
         }
+        double *x = identity ? b : tmp64.ensure((size_t)bn * blk);
+        if (prec == UCFD_PREC_FP64)
+            levels([&](int a, int z) { kexact::pc_lower<double>(blk, a, z, bn, L.P, L.col.p, L.val.p, LU64.p, pm, b, x,
+                                                                0, kind, s); },
+                   [&](int a, int z) { kexact::pc_upper<double>(blk, a, z, bn, U.P, U.col.p, U.val.p, LU64.p, pm, b, x,
+                                                                0, kind, s); });
+        else
+            levels([&](int a, int z) { kfast::pc_lower<double>(blk, a, z, bn, L.P, L.col.p, L.val.p, LU64.p, pm, b, x,
+                                                               0, kind, s); },
+                   [&](int a, int z) { kfast::pc_upper<double>(blk, a, z, bn, U.P, U.col.p, U.val.p, LU64.p, pm, b, x,
+                                                               0, kind, s); });
     }
 };
 

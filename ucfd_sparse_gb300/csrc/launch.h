@@ -96,21 +96,18 @@
     void pc_prepare(int B, int bn, const int *perm, const long long *dslot, const double *values,  \
                     double *LU64, Tl *LU_l, int factor, cudaStream_t s);                           \
     template <typename T>                                                                          \
+    int pc_stride(int B);                                                                          \
+    template <typename T>                                                                          \
     void pc_lower(int B, int t0, int t1, int bn, int PL, const int *Lcol, const T *Lval,           \
-                  const T *LU, T *b, int block, int mode, cudaStream_t s);                         \
+                  const T *LU, const int *perm, double *b, T *x, int block, int mode, cudaStream_t s); \
     template <typename T>                                                                          \
     void pc_upper(int B, int t0, int t1, int bn, int PU, const int *Ucol, const T *Uval,           \
-                  const T *LU, T *b, int block, int mode, cudaStream_t s);                         \
+                  const T *LU, const int *perm, double *b, T *x, int block, int mode, cudaStream_t s); \
     void ilu_factor(int B, int scalar, int t0, int t1, const int *rows, const int *rowptr,         \
                     const int *colidx, const int *diagslots, double *vals, cudaStream_t s);        \
-    template <typename T>                                                                          \
-    void ell_gather(int B, int bn, int P, const int *src, const double *vals, T *out,              \
-                    cudaStream_t s);                                                               \
+    void ell_gather(int B, int bn, int P, const int *src, const double *vals, double *out64,       \
+                    float *out32, cudaStream_t s);                                                 \
     void fingerprint(long long n, const int *a, unsigned long long *out, cudaStream_t s);          \
-    template <typename Ts, typename Td>                                                            \
-    void gather_rows(int bn, int B, const int *perm, const Ts *src, Td *dst, cudaStream_t s);      \
-    template <typename Ts, typename Td>                                                            \
-    void scatter_rows(int bn, int B, const int *perm, const Ts *src, Td *dst, cudaStream_t s);     \
     template <typename Ts, typename Td>                                                            \
     void convert(long long n, const Ts *src, Td *dst, cudaStream_t s);                             \
     template <typename Ts>                                                                         \

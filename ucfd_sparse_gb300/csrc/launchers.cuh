@@ -570,16 +570,27 @@ void bsr_spmv(int B, int bn, int P, const int *col, const Tv *val, double alpha,
     block = spread_block<Ta>(bn, block);
     const unsigned g = grid_for(bn, block);
     const int form = beta == 0.0 ? (alpha == 1.0 ? 1 : 3) : beta == 1.0 && alpha == -1.0 ? 2 : 0;
-    // unrolled rows for the 5x5 systems (tets: diag + 4 faces; hexes: + 6)
+    // unrolled rows for the 5x5 systems (tets: diag + 4 faces; hexes: + 6);
+    // FP32: vector loads of x where its base allows them (rows of 40 bytes)
+    const bool vec = sizeof(Ta) == 4 && ((uintptr_t)x & 15) == 0;
+#define UCFD_SPMV(BB, PW, VEC) \
+    bsr_spmv_kernel<Tv, Ta, BB, PW, VEC><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form)
     if (B == 5 && P <= 5) {
-        bsr_spmv_kernel<Tv, Ta, 5, 5><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form);
+        if constexpr (sizeof(Ta) == 4) {
+            if (vec) return UCFD_SPMV(5, 5, true);
+        }
+        UCFD_SPMV(5, 5, false);
         return;
     }
     if (B == 5 && P <= 7) {
-        bsr_spmv_kernel<Tv, Ta, 5, 7><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form);
+        if constexpr (sizeof(Ta) == 4) {
+            if (vec) return UCFD_SPMV(5, 7, true);
+        }
+        UCFD_SPMV(5, 7, false);
         return;
     }
-    UCFD_KSW(B, (bsr_spmv_kernel<Tv, Ta, BB, 0><<<g, block, 0, s>>>(bn, P, col, val, alpha, x, beta, y, form)));
+    UCFD_KSW(B, (UCFD_SPMV(BB, 0, false)));
+#undef UCFD_SPMV
 }
 
 template <typename Tl>
@@ -591,11 +602,12 @@ void pc_prepare(int B, int bn, const int *perm, const long long *dslot, const do
                                                                              LU_l, factor)));
 }
 
-template <typename T>
-void ell_gather(int B, int bn, int P, const int *src, const double *vals, T *out, cudaStream_t s) {
-    const long long n = (long long)P * bn;
-    if (n <= 0) return;
-    UCFD_KSW(B, (ell_gather_kernel<T, BB><<<grid_for(n), kBlock, 0, s>>>(bn, P, src, vals, out)));
+void ell_gather(int B, int bn, int P, const int *src, const double *vals, double *out64, float *out32,
+                cudaStream_t s) {
+    const long long warps = (long long)P * ((bn + 31) / 32);
+    if (warps <= 0) return;
+    UCFD_KSW(B, (ell_gather_kernel<BB><<<grid_for(warps, kGatherWarps<BB>), 32 * kGatherWarps<BB>, 0, s>>>(
+                    bn, P, src, vals, out64, out32)));
 }
 
 void fingerprint(long long n, const int *a, unsigned long long *out, cudaStream_t s) {
@@ -604,54 +616,58 @@ void fingerprint(long long n, const int *a, unsigned long long *out, cudaStream_
 }
 
 // Triangular steps, mode PC_BLUSGS / PC_BILU / PC_ILU (kernels_krylov.cuh).
+// The working vector x has pc_stride entries per row.
+template <typename T>
+int pc_stride(int B) { return sizeof(T) == 4 && B > 3 ? 8 : B; }
+
+template <typename T, int B, int PW, int MODE, bool LOWER>
+static void pc_kernel_go(unsigned g, int block, cudaStream_t s, int t0, int t1, int bn, int P, const int *col,
+                         const T *val, const T *LU, const int *perm, double *b, T *x) {
+    constexpr int XS = sizeof(T) == 4 && B > 3 ? 8 : B;
+    if constexpr (LOWER)
+        pc_lower_kernel<T, B, PW, MODE, XS><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, perm, b, x);
+    else
+        pc_upper_kernel<T, B, PW, MODE, XS><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, perm, b, x);
+}
+
 template <typename T, int MODE, bool LOWER>
 static void pc_step_go(int B, unsigned g, int block, cudaStream_t s, int t0, int t1, int bn, int P,
-                       const int *col, const T *val, const T *LU, T *b) {
+                       const int *col, const T *val, const T *LU, const int *perm, double *b, T *x) {
     if constexpr (MODE == PC_ILU) {
         if (B != 1) ::ucfd::fail(UCFD_ERR_ARGUMENT, "scalar ILU needs block size 1 (got %d)", B);
-        if constexpr (LOWER) pc_lower_kernel<T, 1, 0, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b);
-        else pc_upper_kernel<T, 1, 0, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b);
+        pc_kernel_go<T, 1, 0, MODE, LOWER>(g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
         return;
     } else {
         if (B == 5 && P <= 6) {
-            if (P <= 4) {
-                if constexpr (LOWER) pc_lower_kernel<T, 5, 4, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b);
-                else pc_upper_kernel<T, 5, 4, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b);
-            } else {
-                if constexpr (LOWER) pc_lower_kernel<T, 5, 6, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b);
-                else pc_upper_kernel<T, 5, 6, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b);
-            }
+            if (P <= 4) pc_kernel_go<T, 5, 4, MODE, LOWER>(g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
+            else pc_kernel_go<T, 5, 6, MODE, LOWER>(g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
             return;
         }
-        if constexpr (LOWER) {
-            UCFD_KSW(B, (pc_lower_kernel<T, BB, 0, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b)));
-        } else {
-            UCFD_KSW(B, (pc_upper_kernel<T, BB, 0, MODE><<<g, block, 0, s>>>(t0, t1, bn, P, col, val, LU, b)));
-        }
+        UCFD_KSW(B, (pc_kernel_go<T, BB, 0, MODE, LOWER>(g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x)));
     }
 }
 
 template <typename T, bool LOWER>
-static void pc_step(int B, int t0, int t1, int bn, int P, const int *col, const T *val, const T *LU, T *b,
-                    int block, int mode, cudaStream_t s) {
+static void pc_step(int B, int t0, int t1, int bn, int P, const int *col, const T *val, const T *LU, const int *perm,
+                    double *b, T *x, int block, int mode, cudaStream_t s) {
     if (t1 <= t0) return;
     block = spread_block<T>(t1 - t0, block);
     const unsigned g = grid_for(t1 - t0, block);
-    if (mode == PC_BILU) pc_step_go<T, PC_BILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, b);
-    else if (mode == PC_ILU) pc_step_go<T, PC_ILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, b);
-    else pc_step_go<T, PC_BLUSGS, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, b);
+    if (mode == PC_BILU) pc_step_go<T, PC_BILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
+    else if (mode == PC_ILU) pc_step_go<T, PC_ILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
+    else pc_step_go<T, PC_BLUSGS, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
 }
 
 template <typename T>
-void pc_lower(int B, int t0, int t1, int bn, int PL, const int *Lcol, const T *Lval, const T *LU, T *b,
-              int block, int mode, cudaStream_t s) {
-    pc_step<T, true>(B, t0, t1, bn, PL, Lcol, Lval, LU, b, block, mode, s);
+void pc_lower(int B, int t0, int t1, int bn, int PL, const int *Lcol, const T *Lval, const T *LU, const int *perm,
+              double *b, T *x, int block, int mode, cudaStream_t s) {
+    pc_step<T, true>(B, t0, t1, bn, PL, Lcol, Lval, LU, perm, b, x, block, mode, s);
 }
 
 template <typename T>
-void pc_upper(int B, int t0, int t1, int bn, int PU, const int *Ucol, const T *Uval, const T *LU, T *b,
-              int block, int mode, cudaStream_t s) {
-    pc_step<T, false>(B, t0, t1, bn, PU, Ucol, Uval, LU, b, block, mode, s);
+void pc_upper(int B, int t0, int t1, int bn, int PU, const int *Ucol, const T *Uval, const T *LU, const int *perm,
+              double *b, T *x, int block, int mode, cudaStream_t s) {
+    pc_step<T, false>(B, t0, t1, bn, PU, Ucol, Uval, LU, perm, b, x, block, mode, s);
 }
 
 // One level of the ILU(0) factorisation (rows[t], t in [t0, t1)).
@@ -665,27 +681,18 @@ void ilu_factor(int B, int scalar, int t0, int t1, const int *rows, const int *r
         ilu_factor_kernel<1, true><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
         return;
     }
-    UCFD_KSW(B, (ilu_factor_kernel<BB, false><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals)));
-}
-
-template <typename Ts, typename Td>
-void gather_rows(int bn, int B, const int *perm, const Ts *src, Td *dst, cudaStream_t s) {
-    const long long n = (long long)bn * B;
-    if (n <= 0) return;
-    gather_rows_kernel<Ts, Td><<<grid_for(n), kBlock, 0, s>>>(bn, B, perm, src, dst);
-}
-
-template <typename Ts, typename Td>
-void scatter_rows(int bn, int B, const int *perm, const Ts *src, Td *dst, cudaStream_t s) {
-    const long long n = (long long)bn * B;
-    if (n <= 0) return;
-    scatter_rows_kernel<Ts, Td><<<grid_for(n), kBlock, 0, s>>>(bn, B, perm, src, dst);
+    if (B > 1) {
+        UCFD_KSW(B, (ilu_factor_rows_kernel<BB><<<grid_for(t1 - t0, 32 / BB), 32, 0, s>>>(t0, t1, rows, rowptr, colidx,
+                                                                                         diagslots, vals)));
+        return;
+    }
+    ilu_factor_kernel<1, false><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
 }
 
 template <typename Ts, typename Td>
 __global__ void convert_kernel(long long n, const Ts *src, Td *dst) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        dst[i] = (Td)src[i];
+        dst[i] = convert_to<Td>(src[i]);
 }
 
 template <typename Ts, typename Td>
@@ -697,7 +704,7 @@ void convert(long long n, const Ts *src, Td *dst, cudaStream_t s) {
 template <typename Ts>
 __global__ void axpy_into_kernel(long long n, const Ts *x, double *y) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        y[i] += (double)x[i];
+        y[i] += to_double(x[i]);
 }
 
 template <typename Ts>
