@@ -148,7 +148,21 @@ static void sweep_lanes_go(const ::ucfd::ScalarSweepArgs<double> &a, int gf, cud
     else UCFD_CUDA(cudaLaunchKernelEx(&cfg, scalar_sweep_lanes_kernel<NV, NFV, NDIMS, SYS, 8>, a));
 }
 
-// Pairs of lanes per cell for a level of this kind, 0: one thread per cell.
+// Larger FP64 levels with rows of at most 8 faces: one thread per active face
+// of a block's cells, whatever the launch variant's register cap.  Up to
+// kPackedMin cells one thread per cell has a sub-partition's FP64 pipe nearly
+// to itself, and the lists' barriers cost more than idle lanes (32^3 cells
+// in two colours of 16384: 191 us a step against 197).
+constexpr int kPackedMin = 16384;
+
+template <int NV, int NFV, int NDIMS, int SYS>
+static void sweep_packed_go(const ::ucfd::ScalarSweepArgs<double> &a, cudaStream_t s) {
+    const unsigned g = grid_for(a.t1 - a.t0, 64);
+    if (a.nface <= 6) scalar_sweep_packed_kernel<NV, NFV, NDIMS, SYS, 6><<<g, 64, 0, s>>>(a);
+    else scalar_sweep_packed_kernel<NV, NFV, NDIMS, SYS, 8><<<g, 64, 0, s>>>(a);
+}
+
+// Pairs of lanes per cell for a level of this kind, 0: another kernel.
 static int sweep_lanes(const ::ucfd::ScalarSweepArgs<double> &a) {
     const long long n = a.t1 - a.t0;
     if (a.pair || a.facelist || a.nface > 8 || n <= 0) return 0;
@@ -165,9 +179,16 @@ void scalar_sweep(const ::ucfd::ScalarSweepArgs<T> &a, int nv, int nfv, int ndim
     if (a.facelist) block = block > 0 ? block : kBlock;
     else block = spread_block<T>(a.pair ? 2ll * (a.t1 - a.t0) : a.t1 - a.t0, block);
     const int gf = sweep_lanes(a);
+    const bool packed = sizeof(T) == 8 && gf == 0 && !a.pair && !a.facelist && a.nface <= 8 &&
+                        a.t1 - a.t0 > kPackedMin;
 #define UCFD_SW(NV, NFV, ND)                                                   \
     if (nv == NV && nfv == NFV && ndims == ND) {                               \
         if constexpr (sizeof(T) == 8) {                                        \
+            if (packed && rans == 0) return sweep_packed_go<NV, NFV, ND, 0>(a, s); \
+            if constexpr (NV > NFV) {                                          \
+                if (packed && rans == 1) return sweep_packed_go<NV, NFV, ND, 1>(a, s); \
+                if (packed) return sweep_packed_go<NV, NFV, ND, 2>(a, s);      \
+            }                                                                  \
             if (gf > 0 && rans == 0) return sweep_lanes_go<NV, NFV, ND, 0>(a, gf, s); \
             if constexpr (NV > NFV) {                                          \
                 if (gf > 0 && rans == 1) return sweep_lanes_go<NV, NFV, ND, 1>(a, gf, s); \
