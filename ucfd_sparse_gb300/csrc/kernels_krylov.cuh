@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int bn, int P, const int 
 
 // Values of a CSR-of-blocks array (row-major B x B blocks in slot order)
 // into the ELL-of-blocks layout: ELL entry (p, k) takes the block at slot
-// src[p*bn + k] (src < 0: padding, zeros), into out64 and / or out32 (rounded
+// src[p*bn + k] (src < 0: padding, not written and never read), into out64 and / or out32 (rounded
 // to FP32) -- one pass for both, since reading the values is half of its
 // traffic.  A warp takes 32 consecutive rows of one p: it reads the blocks
 // one after the other, its lanes along a block (whole sectors instead of one
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps<B>) ell_gather_kernel(int bn
         t[r * LD + j] = qr >= 0 ? __ldg(vals + (long long)qr * B2 + j) : 0.0;
     }
     __syncwarp();
-    if (k >= bn) return;
+    if (q < 0) return;  // padding, or past the last row
     const long long o = (long long)p * B2 * bn + k;
 #pragma unroll
     for (int e = 0; e < B2; ++e) {
