@@ -71,3 +71,44 @@ def test_block_levels_match_the_oracle(m, port, ucfd):
     up, _, res, _ = port.flowsys_blusgs(br, b["rhs"], b["dt"], b["jmat"], b["vol"], b["upts"], nsweeps=2)
     np.testing.assert_array_equal(host(e["upts"]), up)
     np.testing.assert_array_equal(host(e["res"]), res)
+
+
+# either side of the size from which Pack goes through records (131072 cells);
+# 51^3 is no multiple of a warp's 32 cells
+@pytest.mark.parametrize("m", [50, 51])
+@pytest.mark.parametrize("nvars", [5, 7])
+@pytest.mark.parametrize("prec", [0, 2])
+def test_pack_of_large_systems(m, nvars, prec, ucfd):
+    """Two Packs with new inputs, a step after each: elements in an order of
+    their own and in the order of the sweeps give the same cells the same
+    values."""
+    from ucfd_sparse_gb300.flowsys import FlowSys
+    fs = mg.lusgs_flowsys_case(m, nvars=nvars, permute=False)
+    N = fs["nlocal"]
+    c = np.arange(N)
+    color = ((c % m + c // m % m + c // (m * m)) & 1).astype(np.int32)
+    rng = np.random.default_rng(m)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    got = []
+    for order in (np.arange(N), rng.permutation(N)):
+        # element e is cell order[e]; its inputs move with it
+        t = {k: dev(fs[k]) for k in ("rowptr", "colidx", "slots", "sides", "face_area", "face_normal", "rcp_vol")}
+        S = FlowSys(N, nvars, 5, 3, fs["nfaces"], 1, *t.values())
+        S.set_coloring(color)
+        S.set_precision(prec)
+        e = dict(upts=dev(fs["upts"][:, order]), rhs=dev(fs["rhs"][:, order]), dt=dev(fs["dt"][order]),
+                 dsrc=dev(0.1 * np.abs(fs["rhs"][:, order])), vol=dev(fs["vol"][order]))
+        ids = dev(order.astype(np.int32))
+        S.set_element(0, N, 6, ids, e["upts"], e["rhs"], e["dt"], e["dsrc"], e["vol"], torch.zeros_like(e["rhs"]))
+        S.set_lusgs(dev(fs["fspr"]), dev(fs["tfspr"]))
+        for k in range(2):
+            S.lusgs_pack(0, 1.5, 0.3)
+            S.lusgs_run(2, rans=nvars > 5)
+            S.lusgs_update(0)
+            e["rhs"].mul_(-0.5)
+            torch.cuda.synchronize()
+        back = np.empty(N, dtype=np.int64)
+        back[order] = np.arange(N)
+        got.append(e["upts"].cpu().numpy()[:, back])
+    assert np.abs(got[0] - fs["upts"]).max() > 0
+    np.testing.assert_array_equal(got[0], got[1])

@@ -38,6 +38,7 @@ struct Work {
     DevBuf<S> rhs, bdu, dup, J, LU, tJ, tLU;        // block LU-SGS
     DevBuf<S> r, delta;                    // refinement
     DevBuf<S> fl_geo[2];                   // face lists (lower, upper): normal + fa * rv per entry
+    DevBuf<S> rec;                         // Pack's records, one per cell
     DevBuf<S> ulo;                         // FP32 mode: low part of the float-float state u + ulo (UCFDLUSGS_Run)
     DevBuf<S> crhs;                        // fast modes: D^-1 rhs, the block sweeps' right-hand side
     DevBuf<S> spart;                       // each block sweep's own-side sums or terms (SweepSplit)
@@ -108,6 +109,7 @@ struct _FlowSys {
     cudaGraphExec_t run_exec = nullptr;
     int run_rans = -1;
     double run_kappa = 0;
+    int pack_stamp = 0;      // count of Packs that went through records
     bool run_state = false;  // set by UCFDLUSGS_Run, cleared by Pack
     // scalar sweep variant 5: per sweep direction (lower, upper) the active
     // faces cell by cell -- offsets [N + 1], neighbour and ELL slot per entry
@@ -129,6 +131,9 @@ void finish(FlowSys s, bool force_sync = false) {
 // Largest level whose active faces are counted on the host (scalar sweeps of
 // larger levels do not ask).
 constexpr int kActLevel = 16384;
+
+// Cells from which Pack goes through records.
+constexpr long long kPackRecords = 131072;
 
 // Build the level schedule and the ELL mesh arrays (once).
 void build_topology(FlowSys s) {
@@ -1084,10 +1089,29 @@ ucfd_status_t UCFDLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal turb_factor, UCFD
     dispatch(s, [&]<typename S, bool EX>() {
         lusgs_alloc<S>(s);
         Work<S> &w = work<S>(s);
+        if constexpr (std::is_same<S, float>::value) w.ulo.ensure((size_t)s->nvars * s->N);
+        // one element: through records (several elements pack one after the
+        // other into the same arrays, each with its own scattered pass).  Below
+        // this size the scattered writes stay in L2 and one pass is faster.
+        if (s->nelem == 1 && s->N >= kPackRecords) {
+            const bool fresh = w.rec.p == nullptr;
+            S *rec = w.rec.ensure((size_t)kfast::pack_record_words<S>(s->nvars) * s->N);
+            if (fresh) w.rec.zero(w.rec.n, st);  // no stamp from whatever was there
+            if (++s->pack_stamp <= 0) s->pack_stamp = 1;
+            bool ok = false;
+            if constexpr (EX)
+                ok = kexact::fs_lusgs_pack_records<S>(e.neles, s->nvars, s->nfvars, s->N, turb_factor, a0, ids,
+                                                      s->d_iperm.p, up, rh, dt, ds, s->pack_stamp, rec, w.u.p, w.du.p,
+                                                      w.diag.p, w.base.p, w.rhs0.p, w.ulo.p, st);
+            else
+                ok = kfast::fs_lusgs_pack_records<S>(e.neles, s->nvars, s->nfvars, s->N, turb_factor, a0, ids,
+                                                     s->d_iperm.p, up, rh, dt, ds, s->pack_stamp, rec, w.u.p, w.du.p,
+                                                     w.diag.p, w.base.p, w.rhs0.p, w.ulo.p, st);
+            if (ok) return;
+        }
         KCALL(EX, fs_lusgs_pack<S>, e.neles, s->nvars, s->nfvars, s->N, turb_factor, a0, ids, s->d_iperm.p, up, rh,
               dt, ds, w.u.p, w.du.p, w.diag.p, st);
         if constexpr (std::is_same<S, float>::value) {
-            w.ulo.ensure((size_t)s->nvars * s->N);
             kfast::state_lo_pack(e.neles, s->nvars, s->N, ids, s->d_iperm.p, up, w.ulo.p, st);
         }
         const size_t n = (size_t)s->nvars * s->N;

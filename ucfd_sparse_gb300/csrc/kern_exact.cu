@@ -43,4 +43,8 @@ template void pc_lower<double>(int, int, int, int, int, const int *, const doubl
                                double *, double *, int, int, cudaStream_t);
 template void pc_upper<double>(int, int, int, int, int, const int *, const double *, const double *, const int *,
                                double *, double *, int, int, cudaStream_t);
+template int pack_record_words<double>(int);
+template bool fs_lusgs_pack_records<double>(int, int, int, long long, double, double, const int *, const int *,
+                                            const double *, const double *, const double *, const double *, int,
+                                            double *, double *, double *, double *, double *, double *, double *, cudaStream_t);
 }  // namespace kexact

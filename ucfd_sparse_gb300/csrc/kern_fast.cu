@@ -70,4 +70,12 @@ template void axpy_into<float>(long long, const float *, double *, cudaStream_t)
 template void axpy_into<double>(long long, const double *, double *, cudaStream_t);
 template void axpy_norm<double>(long long, const double *, double *, double *, double *, cudaStream_t);
 template void axpy_norm<float>(long long, const float *, float *, double *, double *, cudaStream_t);
+template int pack_record_words<double>(int);
+template bool fs_lusgs_pack_records<double>(int, int, int, long long, double, double, const int *, const int *,
+                                            const double *, const double *, const double *, const double *, int,
+                                            double *, double *, double *, double *, double *, double *, double *, cudaStream_t);
+template int pack_record_words<float>(int);
+template bool fs_lusgs_pack_records<float>(int, int, int, long long, double, double, const int *, const int *,
+                                            const double *, const double *, const double *, const double *, int,
+                                            float *, float *, float *, float *, float *, float *, float *, cudaStream_t);
 }  // namespace kfast

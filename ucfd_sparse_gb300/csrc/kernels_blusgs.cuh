@@ -87,7 +87,7 @@ __device__ __forceinline__ void lusub_dev(const T *LU, T *b) {
     } else {
 #pragma unroll
         for (int row = 1; row < B; ++row) {
-            T v = LU[row * B] * b[0];
+            T v = mul_rn(LU[row * B], b[0]);
 #pragma unroll
             for (int col = 1; col < row; ++col) v += LU[row * B + col] * b[col];
             b[row] -= v;
@@ -96,7 +96,7 @@ __device__ __forceinline__ void lusub_dev(const T *LU, T *b) {
         else b[B - 1] /= LU[B * B - 1];
 #pragma unroll
         for (int row = B - 2; row > -1; --row) {
-            T v = LU[row * B + row + 1] * b[row + 1];
+            T v = mul_rn(LU[row * B + row + 1], b[row + 1]);
 #pragma unroll
             for (int col = row + 2; col < B; ++col) v += LU[row * B + col] * b[col];
             if constexpr (RCP) b[row] = (b[row] - v) * LU[row * B + row];

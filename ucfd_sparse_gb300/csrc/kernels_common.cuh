@@ -55,6 +55,12 @@ __host__ inline int spread_block(long long n, int cap) {
     return want < most ? want : most;
 }
 
+// x * y rounded on its own (never fused into a following add), so that
+// every kernel forms the same term whatever the compiler contracts; with
+// contraction off this is the plain product.
+__device__ __forceinline__ float mul_rn(float x, float y) { return __fmul_rn(x, y); }
+__device__ __forceinline__ double mul_rn(double x, double y) { return __dmul_rn(x, y); }
+
 // (float)x and (double)x on the integer pipe where the value is a normal
 // number of both types or zero: a conversion instruction occupies a SM
 // sub-partition's FP64 pipe for 64 clocks, as long as a multiplication, these

@@ -95,7 +95,7 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
                 const Tv *vp = val + (long long)p * B2 * bn + k;
 #pragma unroll
                 for (int r = 0; r < B; ++r) {
-                    Ta v = (Ta)ld_once<CS>(vp + (long long)(r * B) * bn) * xv[p][0];
+                    Ta v = mul_rn((Ta)ld_once<CS>(vp + (long long)(r * B) * bn), xv[p][0]);
 #pragma unroll
                     for (int cc = 1; cc < B; ++cc) v += (Ta)ld_once<CS>(vp + (long long)(r * B + cc) * bn) * xv[p][cc];
                     if (ZERO && SGN > 0 && p == 0) acc[r] = v;
@@ -116,7 +116,7 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
             const Tv *vp = val + (long long)p * B2 * bn + k;
 #pragma unroll
             for (int r = 0; r < B; ++r) {
-                Ta v = (Ta)ld_once<CS>(vp + (long long)(r * B) * bn) * xv[0];
+                Ta v = mul_rn((Ta)ld_once<CS>(vp + (long long)(r * B) * bn), xv[0]);
 #pragma unroll
                 for (int cc = 1; cc < B; ++cc) v += (Ta)ld_once<CS>(vp + (long long)(r * B + cc) * bn) * xv[cc];
                 if (SGN > 0) acc[r] += v;
@@ -424,14 +424,14 @@ __global__ void __launch_bounds__(32) ilu_factor_rows_kernel(int t0, int t1, con
             x[0] /= lu[0];
 #pragma unroll
             for (int row = 1; row < B; ++row) {
-                double v = x[0] * lu[row];
+                double v = mul_rn(x[0], lu[row]);
 #pragma unroll
                 for (int col = 1; col < row; ++col) v += x[col] * lu[col * B + row];
                 x[row] = (x[row] - v) / lu[row * B + row];
             }
 #pragma unroll
             for (int row = B - 2; row > -1; --row) {
-                double v = x[row + 1] * lu[(row + 1) * B + row];
+                double v = mul_rn(x[row + 1], lu[(row + 1) * B + row]);
 #pragma unroll
                 for (int col = row + 2; col < B; ++col) v += x[col] * lu[col * B + row];
                 x[row] -= v;
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(32) ilu_factor_rows_kernel(int t0, int t1, con
                 double *aij = vals + (long long)jj * B2 + r * B;
 #pragma unroll
                 for (int e = 0; e < B; ++e) {
-                    double v = x[0] * akj[e];
+                    double v = mul_rn(x[0], akj[e]);
 #pragma unroll
                     for (int q = 1; q < B; ++q) v += x[q] * akj[q * B + e];
                     aij[e] -= v;
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(32) ilu_factor_rows_kernel(int t0, int t1, con
 #pragma unroll
         for (int e = k + 1; e < B; ++e) {
             const double u = __shfl_sync(0xffffffffu, d[e], base + k);
-            if (r > k) v[e] = k == 0 ? l * u : v[e] + l * u;
+            if (r > k) v[e] = k == 0 ? mul_rn(l, u) : v[e] + l * u;
         }
         if (r == k + 1) {
 #pragma unroll

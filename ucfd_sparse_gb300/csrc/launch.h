@@ -40,6 +40,14 @@
                        const double *rhs, const double *dt, const double *dsrc, T *u, T *du,       \
                        T *diag, cudaStream_t s);                                                   \
     template <typename T>                                                                          \
+    int pack_record_words(int nvars);                                                              \
+    template <typename T>                                                                          \
+    bool fs_lusgs_pack_records(int neles, int nvars, int nfvars, long long N, double turb_factor,  \
+                               double a0, const int *cell_ids, const int *iperm, const double *upts, \
+                               const double *rhs, const double *dt, const double *dsrc, int stamp, \
+                               T *rec, T *u, T *du, T *diag, T *base, T *rhs0, T *ulo,             \
+                               cudaStream_t s);                                                    \
+    template <typename T>                                                                          \
     void fs_lusgs_update(int neles, int nvars, long long N, const int *cell_ids, const int *iperm, \
                          const T *du, double *upts, int assign, cudaStream_t s);                   \
     template <typename T>                                                                          \

@@ -297,6 +297,33 @@ void fs_lusgs_pack(int neles, int nvars, int nfvars, long long N, double turb_fa
                                                                 du, diag);
 }
 
+// Two-pass Pack (records, then the arrays), nvars 4 .. 7; false: not built for
+// this nvars.  rec holds N records of pack_record_words words.
+template <typename T>
+int pack_record_words(int nvars) { return pack_words<T>(nvars); }
+
+template <typename T>
+bool fs_lusgs_pack_records(int neles, int nvars, int nfvars, long long N, double turb_factor, double a0,
+                           const int *cell_ids, const int *iperm, const double *upts, const double *rhs,
+                           const double *dt, const double *dsrc, int stamp, T *rec, T *u, T *du, T *diag, T *base,
+                           T *rhs0, T *ulo, cudaStream_t s) {
+#define UCFD_PACK(NV)                                                                                            \
+    case NV:                                                                                                     \
+        fs_lusgs_pack_records_kernel<T, NV><<<grid_for(neles), kBlock, 0, s>>>(                                  \
+            neles, nfvars, turb_factor, a0, cell_ids, iperm, upts, rhs, dt, dsrc, stamp, rec);                   \
+        fs_lusgs_unpack_kernel<T, NV><<<grid_for(N, 128), 128, 0, s>>>(N, stamp, rec, u, du, diag, base, rhs0,   \
+                                                                      ulo);                                      \
+        return true;
+    switch (nvars) {
+        UCFD_PACK(4)
+        UCFD_PACK(5)
+        UCFD_PACK(6)
+        UCFD_PACK(7)
+        default: return false;
+    }
+#undef UCFD_PACK
+}
+
 template <typename T>
 void fs_lusgs_update(int neles, int nvars, long long N, const int *cell_ids, const int *iperm,
                      const T *du, double *upts, int assign, cudaStream_t s) {
