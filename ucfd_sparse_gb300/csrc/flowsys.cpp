@@ -358,10 +358,12 @@ void ensure_face_lists(FlowSys s) {
 
 // sys: 0 the mean-flow system, 1 the turbulence system, 2 both in one pass
 // (one thread per cell; the run loop's choice, see run_sweeps_both).
+// own_in: what the swept cells start from (default: their increments).
 // packed: the run loop's sweep of both systems in FP32 reads the packed
 // per cell-face geometry and spectral radii that run_gather_lambda formed.
 template <typename S, bool EX>
-void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent = false, bool packed = false) {
+void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent = false, bool packed = false,
+                 const S *own_in = nullptr) {
     const bool rans = sys == 1;
     Work<S> &w = work<S>(s);
     const long long N = s->N;
@@ -386,7 +388,7 @@ void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent =
     }
     a.u = w.u.p;
     a.nbsrc = w.du.p;
-    a.own_in = w.du.p;
+    a.own_in = own_in ? own_in : w.du.p;
     a.own_out = w.du.p;
     a.diag = w.diag.p;
     a.diag_vs = N;
@@ -607,20 +609,21 @@ template <typename S, bool EX>
 void lusgs_iteration(FlowSys s, bool rans, double kappa, double *resid_slot, bool persistent) {
     Work<S> &w = work<S>(s);
     cudaStream_t st = s->stream();
-    const size_t n = (size_t)s->nvars * s->N;
-    UCFD_CUDA(cudaMemcpyAsync(w.du.p, w.rhs0.p, n * sizeof(S), cudaMemcpyDeviceToDevice, st));
+    // the lower sweeps start from the packed right-hand side itself (a lower
+    // sweep reads no increment that it has not written before): no copy
+    const S *rhs = w.rhs0.p;
     if (rans && run_sweeps_both(s, persistent)) {
         KCALL(EX, fs_lusgs_prepare_both<S>, s->N, s->P, s->nfvars, s->nvars, (S)kappa, s->d_nei.p, geo_fa<S>(s),
               geo_rv<S>(s), w.lamN.p, w.lamT.p, w.base.p, w.diag.p, st);
-        lusgs_sweep<S, EX>(s, 2, false, kappa, persistent, true);
+        lusgs_sweep<S, EX>(s, 2, false, kappa, persistent, true, rhs);
         lusgs_sweep<S, EX>(s, 2, true, kappa, persistent, true);
     } else {
         lusgs_prepare<S, EX>(s, false, kappa, w.base.p);
-        lusgs_sweep<S, EX>(s, 0, false, kappa, persistent);
+        lusgs_sweep<S, EX>(s, 0, false, kappa, persistent, false, rhs);
         lusgs_sweep<S, EX>(s, 0, true, kappa, persistent);
         if (rans) {
             lusgs_prepare<S, EX>(s, true, kappa, w.base.p);
-            lusgs_sweep<S, EX>(s, 1, false, kappa, persistent);
+            lusgs_sweep<S, EX>(s, 1, false, kappa, persistent, false, rhs);
             lusgs_sweep<S, EX>(s, 1, true, kappa, persistent);
         }
     }

@@ -176,12 +176,27 @@ __device__ __forceinline__ void scalar_sweep_cell(const ScalarSweepArgs<T> &a, i
 template <typename T, int NV, int NFV, int NDIMS, bool COHERENT = false, int FB = 3>
 __device__ __forceinline__ void scalar_sweep_cell_both(const ScalarSweepArgs<T> &a, int t, int lo, int hi);
 
+// FP32 sweeps chain the levels' launches: a level starts while the previous
+// one drains, loads what that one does not write (its own inputs, the
+// neighbour indices) and waits here before its first neighbour increment.
+template <typename T>
+__device__ __forceinline__ void wait_for_level(const ScalarSweepArgs<T> &a) {
+    if constexpr (sizeof(T) == 4) {
+        if (a.chained) asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+}
+template <typename T>
+__device__ __forceinline__ void let_next_level_start() {
+    if constexpr (sizeof(T) == 4) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // MINB: minimum resident blocks of 256 threads per SM the compiler must
 // allow (1: no register cap, about 106 registers; 3 / 4: at most 80 / 64
 // registers, more warps to cover the gathers' latency for a few spilled
 // bytes).  The autotuner picks.
 template <typename T, int NV, int NFV, int NDIMS, bool RANS, int MINB = 1>
 __global__ void __launch_bounds__(256, MINB) scalar_sweep_kernel(ScalarSweepArgs<T> a) {
+    let_next_level_start<T>();
     const int t = a.t0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.t1) return;
     scalar_sweep_cell<T, NV, NFV, NDIMS, RANS>(a, t, a.lo, a.hi);
@@ -427,12 +442,14 @@ __device__ __forceinline__ void scalar_sweep_cell(const ScalarSweepArgs<T> &a, i
     // time; the terms are added to df in the reference's face order.
     constexpr int FB = 3, KB = sizeof(T) == 8 ? 1 : FB;
     if (no_active_face(a, lo, hi)) {
+        wait_for_level(a);
     } else if (a.nface <= 2 * FB) {
         // every neighbour index of the cell up front, then its active faces
         int nba[2 * FB];
 #pragma unroll
         for (int p = 0; p < 2 * FB; ++p) nba[p] = p < a.nface ? __ldg(a.nei + p * ld + i) : -1;
         unsigned m = active_faces<T, 2 * FB>(a, lo, hi, ci, nba);
+        wait_for_level(a);
         if constexpr (KB == 1) {
 #pragma unroll 1
             while (m)
@@ -442,6 +459,7 @@ __device__ __forceinline__ void scalar_sweep_cell(const ScalarSweepArgs<T> &a, i
             if (m) face_terms<T, NV, NFV, NDIMS, RANS, COHERENT, 2 * FB, KB, true>(a, i, rvi, 0, nba, m, nullptr, df);
         }
     } else {
+        wait_for_level(a);
         for (int f0 = 0; f0 < a.nface; f0 += FB) {
             int nb[FB];
 #pragma unroll
@@ -543,11 +561,13 @@ __device__ __forceinline__ void scalar_sweep_cell_both(const ScalarSweepArgs<T> 
     }
     const T rvi = a.rv && !a.geo4 ? __ldg(a.rv + i) : T(1);  // packed geometry carries fa * rv
     if (no_active_face(a, lo, hi)) {
+        wait_for_level(a);
     } else if (a.nface <= 2 * FB) {
         int nba[2 * FB];
 #pragma unroll
         for (int p = 0; p < 2 * FB; ++p) nba[p] = p < a.nface ? __ldg(a.nei + p * ld + i) : -1;
         unsigned m = active_faces<T, 2 * FB>(a, lo, hi, ci, nba);
+        wait_for_level(a);
         if constexpr (sizeof(T) == 8) {
 #pragma unroll 1
             while (m) face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, 1>(a, i, rvi, 0, nba, m, df);
@@ -556,6 +576,7 @@ __device__ __forceinline__ void scalar_sweep_cell_both(const ScalarSweepArgs<T> 
             if (m) face_terms_both<T, NV, NFV, NDIMS, COHERENT, 2 * FB, FB>(a, i, rvi, 0, nba, m, df);
         }
     } else {
+        wait_for_level(a);
         for (int f0 = 0; f0 < a.nface; f0 += FB) {
             int nb[FB];
 #pragma unroll
@@ -816,6 +837,7 @@ __global__ void __launch_bounds__(64) scalar_sweep_lanes_kernel(ScalarSweepArgs<
 // are added in face order either way.
 template <typename T, int NV, int NFV, int NDIMS, int MINB = 1>
 __global__ void __launch_bounds__(256, MINB) scalar_sweep_both_kernel(ScalarSweepArgs<T> a) {
+    let_next_level_start<T>();
     const int t = a.t0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.t1) return;
     scalar_sweep_cell_both<T, NV, NFV, NDIMS, false, (MINB >= 3 ? 2 : 3)>(a, t, a.lo, a.hi);

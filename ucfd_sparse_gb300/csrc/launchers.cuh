@@ -77,6 +77,26 @@ void pack_lam2(long long n, const float *lam, const float *tlam, void *lam2, cud
                                                                                    static_cast<float2 *>(lam2));
 }
 
+// A sweep kernel of one level; in FP32 a chained level as a programmatic
+// dependent of the previous one (in FP64 waiting blocks would crowd onto the
+// SMs that run out of work first, see the block sweeps).
+template <typename T>
+static void sweep_launch(void (*kern)(::ucfd::ScalarSweepArgs<T>), const ::ucfd::ScalarSweepArgs<T> &a, long long n,
+                         int block, cudaStream_t s) {
+    ::ucfd::ScalarSweepArgs<T> b = a;
+    if (sizeof(T) == 8) b.chained = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_for(n, block));
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = b.chained ? 1 : 0;
+    UCFD_CUDA(cudaLaunchKernelEx(&cfg, kern, b));
+}
+
 template <typename T, int NV, int NFV, int NDIMS, bool RANS>
 static void sweep_go(const ::ucfd::ScalarSweepArgs<T> &a, int block, cudaStream_t s) {
     const long long n = a.t1 - a.t0;
@@ -98,11 +118,11 @@ static void sweep_go(const ::ucfd::ScalarSweepArgs<T> &a, int block, cudaStream_
         return;
     }
     if (a.regcap == 4)
-        scalar_sweep_kernel<T, NV, NFV, NDIMS, RANS, 4><<<grid_for(n, block), block, 0, s>>>(a);
+        sweep_launch<T>(scalar_sweep_kernel<T, NV, NFV, NDIMS, RANS, 4>, a, n, block, s);
     else if (a.regcap == 3)
-        scalar_sweep_kernel<T, NV, NFV, NDIMS, RANS, 3><<<grid_for(n, block), block, 0, s>>>(a);
+        sweep_launch<T>(scalar_sweep_kernel<T, NV, NFV, NDIMS, RANS, 3>, a, n, block, s);
     else
-        scalar_sweep_kernel<T, NV, NFV, NDIMS, RANS, 1><<<grid_for(n, block), block, 0, s>>>(a);
+        sweep_launch<T>(scalar_sweep_kernel<T, NV, NFV, NDIMS, RANS, 1>, a, n, block, s);
 }
 
 // Both systems in one launch per level (one thread per cell; the register
@@ -114,11 +134,11 @@ static void sweep_both_go(const ::ucfd::ScalarSweepArgs<T> &a, int block, cudaSt
     if (a.facelist || a.pair)
         ::ucfd::fail(UCFD_ERR_UNSUPPORTED, "both-system sweep: one thread per cell only");
     if (a.regcap == 4)
-        scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 4><<<grid_for(n, block), block, 0, s>>>(a);
+        sweep_launch<T>(scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 4>, a, n, block, s);
     else if (a.regcap == 3)
-        scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 3><<<grid_for(n, block), block, 0, s>>>(a);
+        sweep_launch<T>(scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 3>, a, n, block, s);
     else
-        scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 1><<<grid_for(n, block), block, 0, s>>>(a);
+        sweep_launch<T>(scalar_sweep_both_kernel<T, NV, NFV, NDIMS, 1>, a, n, block, s);
 }
 
 // FP64 levels of at most this many cells take scalar_sweep_lanes_kernel: with
