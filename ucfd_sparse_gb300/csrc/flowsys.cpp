@@ -641,10 +641,10 @@ void run_graph_drop(FlowSys s) {
     s->run_exec = nullptr;
 }
 
-// The packed per cell-face geometry and both spectral radii of the FP32
-// sweeps of both systems, from lamN and lamT as just gathered.
+// FP32 sweeps of both systems: the packed per cell-face geometry (fixed with
+// the mesh) and room for both spectral radii; nullptr in FP64.
 template <typename S>
-void pack_both(FlowSys s, cudaStream_t st) {
+void *pack_geo(FlowSys s, cudaStream_t st) {
     if constexpr (std::is_same<S, float>::value) {
         Work<S> &w = work<S>(s);
         const long long nl = (long long)s->P * s->N;
@@ -652,8 +652,17 @@ void pack_both(FlowSys s, cudaStream_t st) {
             w.geo4.ensure((size_t)nl);
             kfast::pack_geo4(s->N, s->P, s->ndims, w.nrm.p, geo_fa<S>(s), geo_rv<S>(s), w.geo4.p, st);
         }
-        w.lam2.ensure((size_t)nl);
-        kfast::pack_lam2(nl, w.lamN.p, w.lamT.p, w.lam2.p, st);
+        return w.lam2.ensure((size_t)nl);
+    }
+    return nullptr;
+}
+
+// And both spectral radii, from lamN and lamT as just gathered.
+template <typename S>
+void pack_both(FlowSys s, cudaStream_t st) {
+    if constexpr (std::is_same<S, float>::value) {
+        Work<S> &w = work<S>(s);
+        kfast::pack_lam2((long long)s->P * s->N, w.lamN.p, w.lamT.p, pack_geo<S>(s, st), st);
         s->lam2_ok = true;
     }
 }
@@ -1173,22 +1182,16 @@ static ucfd_status_t lusgs_prepare_api(FlowSys s, int sys, UCFDReal kappa) {
         Work<S> &w = work<S>(s);
         UCFD_REQUIRE(w.diag.p, "Prepare before Pack");
         const long long nl = (long long)s->P * s->N;
-        if (lfN) {
-            w.lamN.ensure((size_t)nl);
-            kfast::gather_idx<S>(nl, s->d_slot.p, lfN, w.lamN.p, st);
-        }
-        if (lfT) {
-            w.lamT.ensure((size_t)nl);
-            kfast::gather_idx<S>(nl, s->d_slot.p, lfT, w.lamT.p, st);
-        }
+        if (lfN) w.lamN.ensure((size_t)nl);
+        if (lfT) w.lamT.ensure((size_t)nl);
         s->lam2_ok = false;
-        if (sys == 2) {
-            KCALL(EX, fs_lusgs_prepare_both<S>, s->N, s->P, s->nfvars, s->nvars, (S)kappa, s->d_nei.p, geo_fa<S>(s),
-                  geo_rv<S>(s), w.lamN.p, w.lamT.p, (const S *)nullptr, w.diag.p, st);
-            pack_both<S>(s, st);
-        } else {
-            lusgs_prepare<S, EX>(s, sys == 1, kappa, nullptr);
-        }
+        void *lam2 = nullptr;
+        if (sys == 2) lam2 = pack_geo<S>(s, st);
+        KCALL(EX, fs_lusgs_gather_prepare<S>, s->N, s->P, sys == 1 ? s->nfvars : 0, s->nfvars,
+              sys == 0 ? s->nfvars : s->nvars, (S)kappa, s->d_slot.p, geo_fa<S>(s), geo_rv<S>(s),
+              sys == 1 ? lfT : lfN, sys == 2 ? lfT : nullptr, sys == 1 ? w.lamT.p : w.lamN.p, w.lamT.p, lam2,
+              w.diag.p, st);
+        s->lam2_ok = lam2 != nullptr;
     });
     finish(s, (lfN && !is_device_ptr(s->fspr)) || (lfT && !is_device_ptr(s->tfspr)));
     UCFD_API_END

@@ -47,4 +47,7 @@ template int pack_record_words<double>(int);
 template bool fs_lusgs_pack_records<double>(int, int, int, long long, double, double, const int *, const int *,
                                             const double *, const double *, const double *, const double *, int,
                                             double *, double *, double *, double *, double *, double *, double *, cudaStream_t);
+template void fs_lusgs_gather_prepare<double>(long long, int, int, int, int, double, const int *, const double *, const double *,
+                                             const double *, const double *, double *, double *, void *, double *,
+                                             cudaStream_t);
 }  // namespace kexact

@@ -78,4 +78,10 @@ template int pack_record_words<float>(int);
 template bool fs_lusgs_pack_records<float>(int, int, int, long long, double, double, const int *, const int *,
                                             const double *, const double *, const double *, const double *, int,
                                             float *, float *, float *, float *, float *, float *, float *, cudaStream_t);
+template void fs_lusgs_gather_prepare<double>(long long, int, int, int, int, double, const int *, const double *, const double *,
+                                             const double *, const double *, double *, double *, void *, double *,
+                                             cudaStream_t);
+template void fs_lusgs_gather_prepare<float>(long long, int, int, int, int, float, const int *, const float *, const float *,
+                                             const double *, const double *, float *, float *, void *, float *,
+                                             cudaStream_t);
 }  // namespace kfast

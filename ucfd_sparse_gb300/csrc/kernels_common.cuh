@@ -46,10 +46,12 @@ __host__ __device__ inline unsigned grid_for(long long n, int block = kBlock) {
 // blocks of 256: array LU-SGS step of 32^3 cells (two colours of 16384) 250 ->
 // 198 us, natural-order step of 41x36x33 cells (108 levels of at most 1100)
 // 6.44 -> 4.04 ms, both FP64.
+// FP32 levels that fill the SMs take 128 threads (loop of 128^3 cells 8.99 ms
+// with 256, 8.75 with 128, 8.77 with 64); the Krylov kernels ask for 256.
 template <typename T>
 __host__ inline int spread_block(long long n, int cap) {
     constexpr long long kParts = 4 * 152;  // SM sub-partitions
-    const int most = cap > 0 ? cap : (sizeof(T) == 8 ? 64 : 256);
+    const int most = cap > 0 ? cap : (sizeof(T) == 8 ? 64 : 128);
     const long long warps = (n + 31) / 32;
     const int want = warps <= kParts ? 32 : warps <= 4 * kParts ? 64 : most;
     return want < most ? want : most;

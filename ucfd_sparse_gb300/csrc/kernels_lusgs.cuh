@@ -1246,6 +1246,62 @@ __global__ void fs_lusgs_prepare_both_kernel(long long N, int maxdeg, int nfv, i
         for (int v = 0; v < nv; ++v) diag[k + v * N] += v < nfv ? sd : st;
 }
 
+// Prepare of a system (TWO: of both) straight from the face arrays: each cell
+// gathers its faces' spectral radii, leaves the per cell-face copies that the
+// sweeps read (lam, tlam and, where lam2 is given, both packed), and adds the
+// face sums to the diagonal, formed as prepare_sums forms them.  One pass
+// instead of a gather per system, the sums and the packing (113 us for 885K
+// cells FP32, both systems): whole step 455 -> 432 us.
+template <typename T, bool TWO>
+__global__ void __launch_bounds__(256) fs_lusgs_gather_prepare_kernel(long long N, int maxdeg, int nv0, int nfv, int nv1,
+                                                                      T kappa, const int *slot, const T *fa,
+                                                                      const T *rv, const double *lamf,
+                                                                      const double *tlamf, T *lam, T *tlam,
+                                                                      float2 *lam2, T *diag) {
+    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (k >= N) return;
+    T sd = T(0), st = T(0);
+    const T r = rv[k];
+    constexpr int PM = 8;
+    bool live = true;
+    for (int p0 = 0; p0 < maxdeg; p0 += PM) {
+        int s[PM];
+        T f[PM], l[PM], lt[PM];
+#pragma unroll
+        for (int p = 0; p < PM; ++p) {
+            s[p] = p0 + p < maxdeg ? __ldg(slot + (p0 + p) * N + k) : -1;
+            f[p] = p0 + p < maxdeg ? __ldg(fa + (p0 + p) * N + k) : T(0);
+        }
+#pragma unroll
+        for (int p = 0; p < PM; ++p) {
+            l[p] = s[p] >= 0 ? convert_to<T>(__ldg(lamf + s[p])) : T(0);
+            if constexpr (TWO) lt[p] = s[p] >= 0 ? convert_to<T>(__ldg(tlamf + s[p])) : T(0);
+        }
+#pragma unroll
+        for (int p = 0; p < PM; ++p) {
+            if (p0 + p >= maxdeg) break;
+            const long long e = (p0 + p) * N + k;
+            lam[e] = l[p];
+            if constexpr (TWO) {
+                tlam[e] = lt[p];
+                if constexpr (sizeof(T) == 4) {
+                    if (lam2) lam2[e] = make_float2(l[p], lt[p]);
+                }
+            }
+            live = live && s[p] >= 0;
+            if (live) {
+                const T lamf_ = l[p] * kappa;
+                sd += T(0.5) * lamf_ * f[p] * r;
+                if constexpr (TWO) {
+                    const T lamt = lt[p] * kappa;
+                    st += T(0.5) * lamt * f[p] * r;
+                }
+            }
+        }
+    }
+    for (int v = nv0; v < nv1; ++v) diag[k + v * N] += TWO && v >= nfv ? st : sd;
+}
+
 // dst[i] = src[idx[i]] (0 where idx[i] < 0): per cell-face copies of
 // face-indexed arrays.
 template <typename Td>

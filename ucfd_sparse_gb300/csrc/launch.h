@@ -58,6 +58,11 @@
     void fs_lusgs_prepare_both(long long N, int maxdeg, int nfv, int nv, T kappa, const int *nei,  \
                                const T *fa, const T *rv, const T *lam, const T *tlam,              \
                                const T *base, T *diag, cudaStream_t s);                            \
+    template <typename T>                                                                          \
+    void fs_lusgs_gather_prepare(long long N, int maxdeg, int nv0, int nfv, int nv1, T kappa,      \
+                                 const int *slot, const T *fa, const T *rv, const double *lamf,    \
+                                 const double *tlamf, T *lam, T *tlam, void *lam2, T *diag,        \
+                                 cudaStream_t s);                                                  \
     template <typename Td>                                                                         \
     void gather_idx(long long n, const int *idx, const double *src, Td *dst, cudaStream_t s);      \
     void pair_reduce(int nblocks, const double *part, double *out, cudaStream_t s);                \

@@ -367,6 +367,21 @@ void fs_lusgs_prepare_both(long long N, int maxdeg, int nfv, int nv, T kappa, co
                                                                    tlam, base, diag);
 }
 
+template <typename T>
+void fs_lusgs_gather_prepare(long long N, int maxdeg, int nv0, int nfv, int nv1, T kappa, const int *slot, const T *fa,
+                             const T *rv, const double *lamf, const double *tlamf, T *lam, T *tlam, void *lam2,
+                             T *diag, cudaStream_t s) {
+    if (N <= 0) return;
+    const unsigned g = grid_for(N);
+    if (tlamf)
+        fs_lusgs_gather_prepare_kernel<T, true><<<g, kBlock, 0, s>>>(N, maxdeg, nv0, nfv, nv1, kappa, slot, fa, rv, lamf,
+                                                                     tlamf, lam, tlam, static_cast<float2 *>(lam2),
+                                                                     diag);
+    else
+        fs_lusgs_gather_prepare_kernel<T, false><<<g, kBlock, 0, s>>>(N, maxdeg, nv0, nfv, nv1, kappa, slot, fa, rv,
+                                                                      lamf, nullptr, lam, nullptr, nullptr, diag);
+}
+
 template <typename Td>
 void gather_idx(long long n, const int *idx, const double *src, Td *dst, cudaStream_t s) {
     if (n <= 0) return;
@@ -635,7 +650,7 @@ template <typename Tv, typename Ta>
 void bsr_spmv(int B, int bn, int P, const int *col, const Tv *val, double alpha, const double *x,
               double beta, double *y, int block, cudaStream_t s) {
     if (bn <= 0) return;
-    block = spread_block<Ta>(bn, block);
+    block = spread_block<Ta>(bn, block > 0 || sizeof(Ta) == 8 ? block : kBlock);
     const unsigned g = grid_for(bn, block);
     const int form = beta == 0.0 ? (alpha == 1.0 ? 1 : 3) : beta == 1.0 && alpha == -1.0 ? 2 : 0;
     // unrolled rows for the 5x5 systems (tets: diag + 4 faces; hexes: + 6);
@@ -719,7 +734,7 @@ template <typename T, bool LOWER>
 static void pc_step(int B, int t0, int t1, int bn, int P, const int *col, const T *val, const T *LU, const int *perm,
                     double *b, T *x, int block, int mode, cudaStream_t s) {
     if (t1 <= t0) return;
-    block = spread_block<T>(t1 - t0, block);
+    block = spread_block<T>(t1 - t0, block > 0 || sizeof(T) == 8 ? block : kBlock);
     const unsigned g = grid_for(t1 - t0, block);
     if (mode == PC_BILU) pc_step_go<T, PC_BILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
     else if (mode == PC_ILU) pc_step_go<T, PC_ILU, LOWER>(B, g, block, s, t0, t1, bn, P, col, val, LU, perm, b, x);
