@@ -112,3 +112,34 @@ def test_pack_of_large_systems(m, nvars, prec, ucfd):
         got.append(e["upts"].cpu().numpy()[:, back])
     assert np.abs(got[0] - fs["upts"]).max() > 0
     np.testing.assert_array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("m", [4, 25])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_block_sweeps_follow_a_new_right_hand_side(m, prec, ucfd):
+    """A sweep whose first level would only repeat the sweep before is not
+    launched for that level; after a Pack with a new right-hand side, in any
+    direction, it is.  Against the same calls with a Prepare before each sweep
+    (every level and face formed), bit for bit."""
+    from tests.test_gpu_blusgs import make
+    b = mg.blusgs_case(m, permute=False, seed=m + 1)
+    c = np.arange(m ** 3)
+    color = ((c % m + c // m % m + c // (m * m)) & 1).astype(np.int32)
+    got = []
+    for stale in (False, True):
+        S, e = make(b, prec=prec, on_device=True, colored=color)
+        S.blusgs_pack(0, 0.0)
+        S.blusgs_ns_prepare()
+        S.blusgs_reset()
+        for step in "luluPluPulPuluPllu":
+            if step == "P":
+                e["rhs"].mul_(-0.75)
+                torch.cuda.synchronize()
+                S.blusgs_pack(0, 0.0)
+                continue
+            if stale:
+                S.blusgs_ns_prepare()
+            (S.blusgs_ns_lower if step == "l" else S.blusgs_ns_upper)()
+        S.blusgs_update(0)
+        got.append(e["upts"].cpu().numpy())
+    np.testing.assert_array_equal(got[0], got[1])
