@@ -223,8 +223,17 @@ __device__ __forceinline__ double xor_sign(double x, unsigned hi_mask) {
 // (side == 1 ? fv : -fv), the same value bit for bit (a product's sign is
 // the XOR of its operands' signs, its magnitude rounds the same), and the
 // stored off-diagonal value -h0 is a sign-bit flip.
+//
+// Bound by the latency of the record gathers: four blocks of 128 threads per
+// SM (at most 128 registers a thread; without the bound the 5x5 kernel takes
+// more and three are resident).  2.1M hex cells, 5x5, with the transpose:
+// FP32 mode 3991 us without the bound, 3510 with four blocks, 3568 with
+// five, 3679 with six; FMA mode 5617, 5529, 5546, 5558; 64K cells in exact
+// mode 369, 357, 435, 461 (five and six spill).
+constexpr int kPrepareThreads = 128;
+
 template <typename S, int B>
-__global__ void fs_blusgs_prepare_kernel(long long N, int P, const int *nei, const int *slot,
+__global__ void __launch_bounds__(kPrepareThreads, 4) fs_blusgs_prepare_kernel(long long N, int P, const int *nei, const int *slot,
                                          const int8_t *side, const double *fa, const double *rv,
                                          const double *jt, const double *dd, double *D, double *LU64,
                                          S *LU_s, S *J_s, double *J64) {

@@ -442,7 +442,7 @@ void fs_blusgs_prepare(int B, long long N, int P, long long nF, const int *nei, 
     if (N <= 0) return;
     const unsigned gt = (unsigned)((nF + 31) / 32);
     UCFD_BSW(B, (jmat_face_major_kernel<BB><<<gt, 256, 0, s>>>(nF, jmat, jt)));
-    const int block = spread_block<double>(N, 128);
+    const int block = spread_block<double>(N, kPrepareThreads);
     UCFD_BSW(B, (fs_blusgs_prepare_kernel<S, BB><<<grid_for(N, block), block, 0, s>>>(
                     N, P, nei, slot, side, fa, rv, jt, dd, D, LU64, LU_s, J_s, J64)));
 }
