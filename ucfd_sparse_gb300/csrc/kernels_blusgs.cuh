@@ -905,6 +905,10 @@ __global__ void __launch_bounds__(NST == 2 ? 128 : 256)
 // M = D^-1 J fv, so r = rhs - D (x + sum_f M x_nb).
 // Writes r (as R) when r_out != nullptr and accumulates per-block partial
 // sums of r^2 and rhs^2 into part[2*blockIdx.x + {0,1}].
+// Bound by the FP64 pipe (2.1M hex cells, 5x5: 746 us of FP64 instructions
+// and 470 us of reads in 1039 us), so FP32 values are converted with integer
+// instructions (the conversion instruction takes an FP64 slot: 1083 us).
+// More resident blocks change nothing (two to four per SM: 1015 to 1028 us).
 template <typename Sx, typename R, int B>
 __global__ void fs_blusgs_residual_kernel(long long N, int P, int var0, int nvars, const int *nei,
                                           const double *fa, const double *rv, const double *J64,
@@ -918,7 +922,7 @@ __global__ void fs_blusgs_residual_kernel(long long N, int P, int var0, int nvar
         double xk[B];
         // x == nullptr: x is known to be zero, r = rhs (no matrix reads)
 #pragma unroll
-        for (int c = 0; c < B; ++c) xk[c] = x ? (double)x[(var0 + c) * N + k] : 0.0;
+        for (int c = 0; c < B; ++c) xk[c] = x ? to_double(x[(var0 + c) * N + k]) : 0.0;
         // M form: t = x + sum_f M x_nb, then r = rhs - D t (below)
         double t[B];
 #pragma unroll
@@ -947,7 +951,7 @@ __global__ void fs_blusgs_residual_kernel(long long N, int P, int var0, int nvar
             for (int q = 0; q < PU; ++q) {
                 const int g = nbv[q] >= 0 ? nbv[q] : (int)k;
 #pragma unroll
-                for (int c = 0; c < B; ++c) xn[q][c] = (double)x[(var0 + c) * N + g];
+                for (int c = 0; c < B; ++c) xn[q][c] = to_double(x[(var0 + c) * N + g]);
             }
 #pragma unroll
             for (int q = 0; q < PU; ++q) {
@@ -974,7 +978,7 @@ __global__ void fs_blusgs_residual_kernel(long long N, int P, int var0, int nvar
 #pragma unroll
         for (int r = 0; r < B; ++r) {
             rr += res[r] * res[r];
-            if (r_out) r_out[(var0 + r) * N + k] = (R)res[r];
+            if (r_out) r_out[(var0 + r) * N + k] = convert_to<R>(res[r]);
         }
     }
     rr = block_sum(rr);
