@@ -148,7 +148,8 @@ UCFD_EXTERN ucfd_status_t UCFDFlowSysSetStream(FlowSys sys, void *cuda_stream, i
 
 /* Scalar LU-SGS pseudo-time loop on device-resident state: niter times
  * { du = rhs; NS prepare; NS lower; NS upper; [RANS prepare/lower/upper];
- *   u += du }, launched as one CUDA graph (mode 0) or as one persistent
+ *   u += du } -- the diagonals, which do not depend on u, are prepared once
+ * per call, with the values every iteration would give -- launched as one CUDA graph (mode 0) or as one persistent
  * grid-synchronised kernel per sweep (mode 1); mode -1 takes the run_mode
  * of the launch configuration (UCFDFlowSysAutotune).  Requires a prior Pack of
  * every element.  resid (optional, [niter]) receives sqrt(sum du^2)
