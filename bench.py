@@ -35,9 +35,9 @@ METRIC = "LU-SGS cell-updates/s & HBM GB/s @2.1M cells; FP32+refine vs FP64 @1e-
 UNIT = "cell-updates/s"
 # DRAM bytes per cell update of the unrolled FP32 block sweep: ncu
 # dram__bytes_read.sum + dram__bytes_write.sum over one lower + upper sweep
-# pair on the 96^3 mesh (718.1 MB for 2 x 884,736 cell updates;
+# pair on a 96^3 mesh (691.8 MB for 2 x 884,736 cell updates;
 # profiles/fs_blusgs_sweep_96cubed.md)
-SWEEP_TRAFFIC_PER_CELL = 405.8
+SWEEP_TRAFFIC_PER_CELL = 391.0
 
 
 # ---------------------------------------------------------------------------
@@ -248,7 +248,9 @@ def launches_per_step(nlev, pairs, inner, mixed):
     outer = math.ceil(pairs / inner) if pairs else 0
     n = 1 + 2 + 1                                  # pack, prepare (jmat transpose + diagonal/LU), update
     n += 2                                         # initial residual + reduction
-    n += outer * 2 + pairs * 2 * nlev              # residual per outer loop, sweeps
+    # residual per outer loop; sweeps, which leave out their first level unless
+    # the increments were just set (each outer loop's first lower sweep)
+    n += outer * 2 + pairs * 2 * (nlev - 1) + outer
     if mixed:
         n += 2 + 2 * outer                         # conversions; per outer step x += delta and D^-1 r
     return n
@@ -524,28 +526,35 @@ def run_gpu(args):
     except OSError:
         pass
     peak = float(peaks.get("hbm_gbs", 6800.0))
-    bytes_sweep64 = sweep_bytes(case["rowptr"], 8, 5)
-    bytes_sweep = sweep_bytes(case["rowptr"], 4, 5)
+    # a sweep after a sweep leaves out its first level (first colour of a lower
+    # sweep, last of an upper one): its cells' indices and vectors do not move
+    sizes = np.bincount(np.asarray(lc))
+    sizes = sizes[sizes > 0]
+    left_out = (int(sizes[0]) + int(sizes[-1])) / 2
+    row = int(case["rowptr"][-1]) / N
+    bytes_sweep64 = sweep_bytes(case["rowptr"], 8, 5) - left_out * (4 * row + 5 * 5 * 8)
+    bytes_sweep = sweep_bytes(case["rowptr"], 4, 5) - left_out * (4 * row + 5 * 5 * 4)
+    nlaunch = max(nlev - 1, 1)
     achieved = bytes_sweep / (sweep_ms * 1e-3) / 1e9
-    launch_bytes = bytes_sweep / nlev
+    launch_bytes = bytes_sweep / nlaunch
     cfg32 = P32.S.launch_config()
     kname = {0: "fs_blusgs_sweep_kernel<float,5,6>", 1: "fs_blusgs_sweep_kernel<float,5,0>",
              2: "fs_blusgs_sweep_bulk_kernel<5,6,2>", 3: "fs_blusgs_sweep_bulk_kernel<5,6,1>",
-             4: "fs_blusgs_sweep_kernel<float,5,6,true>"}.get(cfg32["sweep_variant"], "fs_blusgs_sweep_kernel")
+             4: "fs_blusgs_sweep_kernel<float,5,6>", 5: "fs_blusgs_sweep_kernel<float,5,6>"}.get(cfg32["sweep_variant"], "fs_blusgs_sweep_kernel")
     # DRAM bytes per cell update from ncu (dram__bytes_read.sum + write) of
     # the unrolled FP32 sweep on the 64^3 case, scaled to this launch's cells
-    traffic = (SWEEP_TRAFFIC_PER_CELL * N / nlev if SWEEP_TRAFFIC_PER_CELL and cfg32["sweep_variant"] in (0, 4)
+    traffic = (SWEEP_TRAFFIC_PER_CELL * N / nlaunch if SWEEP_TRAFFIC_PER_CELL and cfg32["sweep_variant"] in (0, 4, 5)
                else None)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "kernel": kname, "threads_per_block": cfg32["threads_per_block"],
-                "algorithmic_bytes_per_launch": launch_bytes, "launch_ms": sweep_ms / nlev,
+                "algorithmic_bytes_per_launch": launch_bytes, "launch_ms": sweep_ms / nlaunch,
                 "traffic_source": f"ncu 96^3 capture of a sweep pair, {SWEEP_TRAFFIC_PER_CELL} B per cell update, "
                                   "scaled by cells per launch",
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if peaks else "fallback 6.8 TB/s",
                 "pair_ms": 2 * sweep_ms,
                 "algorithmic_bytes_per_cell_update": bytes_sweep / N,
                 "bytes_note": "split-sum sweeps: every neighbour index each sweep, each face block once per "
-                              "lower+upper pair (in the sweep that updates its side), 5 vectors per cell"}
+                              "lower+upper pair (in the sweep that updates its side), 5 vectors per swept cell"}
 
     # ---- error of one step against the FP64 arithmetic of the oracle --------
     # (UCFD_PREC_FP64 runs the reference's operation order, bit-identical to
@@ -659,7 +668,7 @@ def run_gpu(args):
                      "value": N * statistics.mean(pairs64) / (ms64 * 1e-3),
                      "sweep_ms": sweep64_ms, "sweep_GBps": bytes_sweep64 / (sweep64_ms * 1e-3) / 1e9,
                      "sweep_frac": bytes_sweep64 / (sweep64_ms * 1e-3) / 1e9 / peak,
-                     "sweep_kernel": "fs_blusgs_sweep_kernel<double,5,6,true> (FP64 with fused multiply-adds)"},
+                     "sweep_kernel": "fs_blusgs_sweep_kernel<double,5,6> (FP64 with fused multiply-adds)"},
             "speedup_fp32_refined_vs_fp64": ms64 / ms32,
             "err_vs_fp64": err["err_vs_fp64"], "error": err,
             "roofline": roofline,
@@ -689,27 +698,23 @@ def _events(stream):
 
 def lusgs_iter_bytes(rowptr, elt, nfv=5, nt=1, both=False):
     """Algorithmic bytes of one scalar LU-SGS pseudo-time iteration per
-    UCFDLUSGS_Run (NS + RANS prepare, lower and upper sweeps, update), FlowSys
-    layout: per face its index, area, spectral radius and (once, in the sweep
-    where it is active) its normal; per cell the packed diagonal, the state
-    and increment of every variable read/written once.  both: the loop's
-    one-pass kernels (one prepare and one sweep per direction for both
-    systems), which read each face's index and area once per kernel."""
+    UCFDLUSGS_Run (NS + RANS lower and upper sweeps, update; the diagonals are
+    prepared once per loop), FlowSys layout: per face its index, area, spectral
+    radius and (once, in the sweep where it is active) its normal; per cell the
+    diagonal, the right-hand side, the state and increment of every variable
+    read/written once.  both: the loop's one-pass kernels (one sweep per
+    direction for both systems), which read each face's index and area once
+    per kernel."""
     nnz = int(rowptr[-1])
     N = rowptr.shape[0] - 1
     nv = nfv + nt
     if both:
-        per_face = (4 + 3 * elt) + 2 * (4 + 3 * elt) + 3 * elt    # prepare, 2 sweeps, normal once
-        per_cell = 2 * nv * elt                                    # du = rhs copy
-        per_cell += elt + 2 * nv * elt                             # rcp_vol, diag from base
-        per_cell += 2 * (elt + nfv * elt + 3 * nv * elt)           # sweeps: rv, u, du own r/w + nbr, diag
+        per_face = 2 * (4 + 3 * elt) + 3 * elt                     # 2 sweeps, normal once
+        per_cell = 2 * (elt + nfv * elt + 3 * nv * elt)           # sweeps: rv, u, du own r/w + nbr, diag
         per_cell += 3 * nv * elt                                   # u += du
         return nnz * per_face + N * per_cell
-    per_face = (4 + 2 * elt) * 2 + (4 + 3 * elt + 2 * elt)   # NS prepare + sweeps
-    per_face += (4 + 2 * elt) + (4 + 3 * elt + 2 * elt)      # RANS prepare + sweeps
-    per_cell = 2 * nv * elt                                    # du = rhs copy
-    per_cell += elt + 2 * nfv * elt + elt + 2 * nt * elt       # rcp_vol, diag from base (NS, RANS)
-    per_cell += 2 * (elt + 5 * elt + 3 * nfv * elt)            # NS sweeps: rv, u, du own r/w + nbr, diag
+    per_face = 2 * ((4 + 2 * elt) + (4 + 3 * elt + 2 * elt))  # NS, RANS sweeps
+    per_cell = 2 * (elt + 5 * elt + 3 * nfv * elt)            # NS sweeps: rv, u, du own r/w + nbr, diag
     per_cell += 2 * (elt + 5 * elt + 3 * nt * elt)             # RANS sweeps
     per_cell += 3 * nv * elt                                   # u += du
     return nnz * per_face + N * per_cell
