@@ -98,6 +98,8 @@ struct _FlowSys {
     DevBuf<double> jt;  // Prepare scratch: face Jacobians, one record per face
     DevBuf<int> d_sweep_err;  // set by a bulk-copy block sweep whose copy wait gave up
     bool bulk_swept = false;  // a bulk-copy variant ran since d_sweep_err was last read
+    bool captured = false;    // a caller captured block sweeps into a graph: it may replay them at any time
+    bool bulk_captured = false;  // ... with a bulk-copy variant
     bool du64_valid = false;
     bool c_valid[2] = {false, false};  // crhs of the NS / turbulence rows matches rhs and the factors
     bool x_zero = false;  // the correction du is all zeros (Reset, no sweep since)
@@ -489,7 +491,7 @@ void blusgs_alloc(FlowSys s) {
 // Only those variants (2 and 3) wait for a copy; after the others there is
 // nothing to read, which saves a copy and a second synchronisation per call.
 void check_sweep_err(FlowSys s) {
-    if (!s->d_sweep_err.p || !s->bulk_swept) return;
+    if (!s->d_sweep_err.p || !(s->bulk_swept || s->bulk_captured)) return;
     s->bulk_swept = false;
     int err = 0;
     UCFD_CUDA(cudaMemcpyAsync(&err, s->d_sweep_err.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream()));
@@ -527,6 +529,17 @@ const S *sweep_rhs(FlowSys s, bool turb) {
     return w.crhs.p;
 }
 
+// Whether the caller is capturing the handle's stream: the call's work runs
+// when (and as often as) the graph is launched, not now.
+bool capturing(FlowSys s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream(), &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 template <typename S, bool EX>
 void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     Work<S> &w = work<S>(s);
@@ -545,13 +558,21 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0]) ? 0 : 1;
     const S *fa = geo_fa<S>(s);
     if constexpr (EX) fa = s->fv64.p;
-    if (s->variant == 2 || s->variant == 3) s->bulk_swept = true;
+    // What the host knows of the increments and the stored terms ends where
+    // sweeps run from a captured graph: from then on no sweep leaves out a
+    // level, and the exact mode forms every term in every sweep.
+    s->captured = s->captured || capturing(s);
+    if (EX && s->captured) sp.full = 1;
+    if (s->variant == 2 || s->variant == 3) {
+        s->bulk_swept = true;
+        s->bulk_captured = s->bulk_captured || s->captured;
+    }
     // The first level of a sweep has no face towards an earlier one: all it
     // uses are the other side's sums or terms, as the sweep before formed them
     // with this right-hand side, and it would write the increments that sweep
     // left (the largest colour in a lower sweep: 22 of 389 us per pair at 226K
     // cells FP64, and the last colour's launch in an upper one).
-    const bool settled = !sp.full && ss.rhs == rhs && ss.rver == s->rver;
+    const bool settled = !sp.full && !s->captured && ss.rhs == rhs && ss.rver == s->rver;
     // The last level has no face towards a later one: it need not (and, its
     // own sums of the sweep that skipped it still in place, must not) read
     // the other side.
@@ -1136,7 +1157,8 @@ ucfd_status_t UCFDLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal turb_factor, UCFD
         // one element: through records (several elements pack one after the
         // other into the same arrays, each with its own scattered pass).  Below
         // this size the scattered writes stay in L2 and one pass is faster.
-        if (s->nelem == 1 && s->N >= kPackRecords) {
+        // (Not into a graph, whose every launch would write the same stamp.)
+        if (s->nelem == 1 && s->N >= kPackRecords && !capturing(s)) {
             const bool fresh = w.rec.p == nullptr;
             S *rec = w.rec.ensure((size_t)kfast::pack_record_words<S>(s->nvars) * s->N);
             if (fresh) w.rec.zero(w.rec.n, st);  // no stamp from whatever was there
