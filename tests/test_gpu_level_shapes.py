@@ -191,3 +191,52 @@ def test_captured_sweeps(m, prec, ucfd):
         torch.cuda.synchronize()
         got.append(e["upts"].cpu().numpy())
     np.testing.assert_array_equal(got[0], got[1])
+
+
+# a square of m x m cells in two colours: levels of 32, 12168 (lanes), 12800
+# (one thread per cell) and 17298 cells (one thread per active face) in FP64
+@pytest.mark.parametrize("m", [8, 156, 160, 186])
+@pytest.mark.parametrize("nvars", [4, 5, 6])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_plane_levels(m, nvars, prec, ucfd):
+    """Two-dimensional cells: the kernels chosen by the level's size and two
+    threads per cell (variant 3) agree bit for bit."""
+    from ucfd_sparse_gb300.flowsys import FlowSys
+    rng = np.random.default_rng(m)
+    N = m * m
+    c = np.arange(N)
+    x, y = c % m, c // m
+    right, up = c[x < m - 1], c[y < m - 1]
+    a, b = np.concatenate([right, up]), np.concatenate([right + 1, up + m])
+    nF = a.size
+    row, col = np.concatenate([a, b]), np.concatenate([b, a])
+    slot, side = np.tile(np.arange(nF), 2), np.repeat([1, -1], nF)
+    k = np.lexsort((rng.random(2 * nF), row))
+    rowptr = np.searchsorted(row[k], np.arange(N + 1)).astype(np.int32)
+    ang = rng.uniform(0, 2 * np.pi, nF)
+    upts = np.empty((nvars, N))
+    upts[:4] = np.array([1.0, 0.4, -0.2, 2.5])[:, None] * rng.uniform(0.95, 1.05, (4, N))
+    upts[4:] = rng.uniform(0.1, 1.0, (nvars - 4, N))
+    dev = lambda v: torch.from_numpy(np.ascontiguousarray(v)).cuda()  # noqa: E731
+    rhs, dt = rng.standard_normal((nvars, N)) * 1e-2, rng.uniform(1e-3, 1e-2, N)
+    got = []
+    for variant in (0, 3):
+        t = [dev(v) for v in (rowptr, col[k].astype(np.int32), slot[k].astype(np.int32), side[k].astype(np.int8),
+                              1.25 + 0.5 * np.sin(ang), np.stack([np.cos(ang), np.sin(ang)], 1),
+                              1.0 / (1.0 + 0.1 * x / m))]
+        S = FlowSys(N, nvars, 4, 2, nF, 1, *t)
+        S.set_coloring(((x + y) & 1).astype(np.int32))
+        S.set_precision(prec)
+        S.set_launch_config(sweep_variant=variant)
+        e = [dev(v) for v in (upts, rhs, dt, np.zeros((nvars, N)), np.ones(N), np.zeros((nvars, N)))]
+        ids = dev(c.astype(np.int32))
+        S.set_element(0, N, 4, ids, *e)
+        f = dev(1.0 + 0.5 * np.sin(np.arange(nF))), dev(1.0 + 0.5 * np.cos(np.arange(nF)))
+        S.set_lusgs(*f)
+        S.lusgs_pack(0, 1.5, 0.3)
+        S.lusgs_run(2, rans=nvars > 4)
+        S.lusgs_update(0)
+        torch.cuda.synchronize()
+        got.append(e[0].cpu().numpy())
+    assert np.isfinite(got[0]).all() and not np.array_equal(got[0], upts)
+    np.testing.assert_array_equal(got[0], got[1])
