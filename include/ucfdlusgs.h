@@ -143,16 +143,27 @@ UCFD_EXTERN ucfd_status_t UCFDFlowSysGetLaunchConfig(FlowSys sys, UCFDLaunchConf
 UCFD_EXTERN ucfd_status_t UCFDFlowSysSetLaunchConfig(FlowSys sys, const UCFDLaunchConfig *cfg);
 /* Run all kernels of a call on the caller's CUDA stream and return without
  * synchronising (stream == NULL restores the private stream and synchronous
- * calls).  Host-pointer arguments still synchronise. */
+ * calls).  Host-pointer arguments still synchronise.
+ *
+ * Calls on such a stream can be captured into a CUDA graph of the caller's
+ * (device-pointer arguments; each kind of call made once before, since first
+ * calls allocate).  A launched graph does what its calls would do at that
+ * place.  Block LU-SGS sweeps read back face sums or terms of the sweep before
+ * only where both are in the same capture, or neither is and nothing was
+ * captured before: the graph may run between any two calls, so once block
+ * calls of a handle have been captured, its uncaptured sweeps form every face
+ * (for as long as the handle lives; Solve keeps them within its own call).
+ * UCFD_PREC_FP32: an Update captured without a sweep before it in the same
+ * graph adds the FP32 increments, also after a Solve. */
 UCFD_EXTERN ucfd_status_t UCFDFlowSysSetStream(FlowSys sys, void *cuda_stream, int async);
 
 /* Scalar LU-SGS pseudo-time loop on device-resident state: niter times
  * { du = rhs; NS prepare; NS lower; NS upper; [RANS prepare/lower/upper];
  *   u += du } -- the diagonals, which do not depend on u, are prepared once
- * per call, with the values every iteration would give -- launched as one CUDA graph (mode 0) or as one persistent
- * grid-synchronised kernel per sweep (mode 1); mode -1 takes the run_mode
- * of the launch configuration (UCFDFlowSysAutotune).  Requires a prior Pack of
- * every element.  resid (optional, [niter]) receives sqrt(sum du^2)
+ * per call, with the values every iteration would give -- launched as one
+ * CUDA graph (mode 0) or as one persistent grid-synchronised kernel per
+ * sweep (mode 1); mode -1 takes the run_mode of the launch configuration
+ * (UCFDFlowSysAutotune).  Requires a prior Pack of every element.  resid (optional, [niter]) receives sqrt(sum du^2)
  * accumulated to FP64 accuracy after each iteration.  Update() afterwards
  * writes the final state back to the element arrays.  With UCFD_PREC_FP32
  * the sweeps read the FP32 state while u += du accumulates into a

@@ -58,6 +58,7 @@ struct SplitState {
     // changes); null when du was set to zero instead of swept
     const void *rhs = nullptr;
     unsigned rver = 0;
+    unsigned long long capture = 0;  // the capture (capture_id) that sweep was part of; 0: it ran when called
 };
 
 }  // namespace
@@ -98,10 +99,17 @@ struct _FlowSys {
     DevBuf<double> jt;  // Prepare scratch: face Jacobians, one record per face
     DevBuf<int> d_sweep_err;  // set by a bulk-copy block sweep whose copy wait gave up
     bool bulk_swept = false;  // a bulk-copy variant ran since d_sweep_err was last read
-    bool captured = false;    // a caller captured block sweeps into a graph: it may replay them at any time
+    // A caller captured calls of the block path into a graph, which may run
+    // between any two calls from then on: what the host noted of the device's
+    // state (split, c_valid, x_zero) holds within one capture, in the order of
+    // the graph, and within one call (in_call), and no longer.
+    bool captured = false;
+    bool in_call = false;
     bool bulk_captured = false;  // ... with a bulk-copy variant
     bool du64_valid = false;
+    DevBuf<int> d_du_newer;  // FP32: set by a captured sweep that ran, whose du x64 then no longer holds
     bool c_valid[2] = {false, false};  // crhs of the NS / turbulence rows matches rhs and the factors
+    unsigned long long c_capture[2] = {0, 0};  // the capture that formed it (as SplitState::capture)
     bool x_zero = false;  // the correction du is all zeros (Reset, no sweep since)
     SplitState split[2];           // NS / turbulence rows of the fast block sweeps
     unsigned jver[2] = {1, 1};     // Prepare count of the NS / turbulence blocks
@@ -484,6 +492,7 @@ void blusgs_alloc(FlowSys s) {
         if (std::is_same<S, float>::value) w.tLU.ensure(tiled_size(N, t2));
     }
     if (!s->d_sweep_err.p) s->d_sweep_err.zero(1, s->stream());
+    if (std::is_same<S, float>::value && !s->d_du_newer.p) s->d_du_newer.zero(1, s->stream());
 }
 
 // Bulk-copy sweeps report a copy wait that gave up through d_sweep_err;
@@ -511,33 +520,50 @@ const S *blu_LU(FlowSys s, bool turb) {
     else return turb ? s->w32.tLU.p : s->w32.LU.p;
 }
 
+// The capture that the handle's stream is under: the call's work then runs
+// when (and as often as) the graph is launched, not now.  0: none.
+unsigned long long capture_id(FlowSys s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(s->stream(), &st, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return ~0ull;
+    }
+    return st == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
+// The same for a call of the block path, which notes that there is one.
+unsigned long long block_capture_id(FlowSys s) {
+    const unsigned long long id = capture_id(s);
+    s->captured = s->captured || id != 0;
+    return id;
+}
+
+// Whether what a call under capture `then` left on the device is still there
+// for a call under capture `now`.
+bool still_holds(FlowSys s, unsigned long long then, unsigned long long now) {
+    return then == now && (now != 0 || !s->captured || s->in_call);
+}
+
 // Right-hand side of the fast modes' block sweeps (their blocks are
 // M = D^-1 J fv, so a sweep starts from D^-1 rhs): computed from the packed
-// rhs when Pack or Prepare changed it; the exact mode sweeps rhs itself.
+// rhs when Pack or Prepare changed it, or a graph may have; the exact mode
+// sweeps rhs itself.
 template <typename S, bool EX>
 const S *sweep_rhs(FlowSys s, bool turb) {
     Work<S> &w = work<S>(s);
     if constexpr (EX) return w.rhs.p;
     const int B = turb ? s->ntvars : s->nfvars;
     const int var0 = turb ? s->nfvars : 0;
-    if (!s->c_valid[turb ? 1 : 0]) {
+    const unsigned long long now = block_capture_id(s);
+    if (!s->c_valid[turb ? 1 : 0] || !still_holds(s, s->c_capture[turb ? 1 : 0], now)) {
         w.crhs.ensure((size_t)s->nvars * s->N);
         kfast::fs_blusgs_rhs_solve<S>(B, s->N, var0, blu_LU<S>(s, turb), w.rhs.p, w.crhs.p, s->stream());
         s->c_valid[turb ? 1 : 0] = true;
+        s->c_capture[turb ? 1 : 0] = now;
         ++s->rver;
     }
     return w.crhs.p;
-}
-
-// Whether the caller is capturing the handle's stream: the call's work runs
-// when (and as often as) the graph is launched, not now.
-bool capturing(FlowSys s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s->stream(), &st) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
-    return st != cudaStreamCaptureStatusNone;
 }
 
 template <typename S, bool EX>
@@ -555,24 +581,21 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     sp.part = w.spart.ensure((size_t)(EX ? s->P : 1) * s->nvars * s->N);
     sp.upper = upper ? 1 : 0;
     sp.nvars = s->nvars;
-    sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0]) ? 0 : 1;
+    const unsigned long long now = block_capture_id(s);
+    sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0] &&
+               still_holds(s, ss.capture, now)) ? 0 : 1;
     const S *fa = geo_fa<S>(s);
     if constexpr (EX) fa = s->fv64.p;
-    // What the host knows of the increments and the stored terms ends where
-    // sweeps run from a captured graph: from then on no sweep leaves out a
-    // level, and the exact mode forms every term in every sweep.
-    s->captured = s->captured || capturing(s);
-    if (EX && s->captured) sp.full = 1;
     if (s->variant == 2 || s->variant == 3) {
         s->bulk_swept = true;
-        s->bulk_captured = s->bulk_captured || s->captured;
+        s->bulk_captured = s->bulk_captured || now != 0;
     }
     // The first level of a sweep has no face towards an earlier one: all it
     // uses are the other side's sums or terms, as the sweep before formed them
     // with this right-hand side, and it would write the increments that sweep
     // left (the largest colour in a lower sweep: 22 of 389 us per pair at 226K
     // cells FP64, and the last colour's launch in an upper one).
-    const bool settled = !sp.full && !s->captured && ss.rhs == rhs && ss.rver == s->rver;
+    const bool settled = !sp.full && ss.rhs == rhs && ss.rver == s->rver;
     // The last level has no face towards a later one: it need not (and, its
     // own sums of the sweep that skipped it still in place, must not) read
     // the other side.
@@ -584,7 +607,7 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
               s->block, s->variant, s->d_sweep_err.p, kBulkMaxSpin, sp, s->stream());
         if (s->sch.lev_off[l + 1] > s->sch.lev_off[l]) sp.chained = 1;
     }
-    ss = SplitState{du, upper ? 1 : 0, s->jver[turb ? 1 : 0], rhs, s->rver};
+    ss = SplitState{du, upper ? 1 : 0, s->jver[turb ? 1 : 0], rhs, s->rver, now};
 }
 
 // du of the fast block sweeps was set to zero: both sides' sums are zero,
@@ -596,10 +619,32 @@ void split_zero(FlowSys s, bool turb, const S *du, cudaStream_t st) {
     const int var0 = turb ? s->nfvars : 0;
     w.spart.ensure((size_t)s->nvars * s->N);
     UCFD_CUDA(cudaMemsetAsync(w.spart.p + (size_t)var0 * s->N, 0, (size_t)B * s->N * sizeof(S), st));
-    s->split[turb ? 1 : 0] = SplitState{du, 1, s->jver[turb ? 1 : 0], nullptr, 0};
+    s->split[turb ? 1 : 0] = SplitState{du, 1, s->jver[turb ? 1 : 0], nullptr, 0, block_capture_id(s)};
 }
 
 void split_forget(FlowSys s) { s->split[0] = s->split[1] = SplitState{}; }
+
+// Sweeps that one call makes one after the other: no graph runs in between.
+struct InCall {
+    FlowSys s;
+    explicit InCall(FlowSys h) : s(h) {
+        if (s->captured) {
+            split_forget(s);
+            s->c_valid[0] = s->c_valid[1] = false;
+        }
+        s->in_call = true;
+    }
+    ~InCall() { s->in_call = false; }
+};
+
+// FP32, x64 in use (du64_valid): du of a captured sweep that ran since takes
+// its place.
+void x64_from_du(FlowSys s) {
+    if (s->captured && s->du64_valid)
+        kfast::widen_if((long long)s->nvars * s->N, s->d_du_newer.p, s->w32.bdu.p, s->x64.p, s->stream());
+}
+
+bool x_is_zero(FlowSys s) { return s->x_zero && !s->captured; }
 
 // FP64 residual of the NS block system for x; returns ||r|| and ||rhs||.
 template <typename Sx, typename R, bool EX>
@@ -1006,6 +1051,7 @@ ucfd_status_t UCFDFlowSysAutotune(FlowSys s, int reps, UCFDLaunchConfig *best) {
             UCFD_REQUIRE(w.rhs.p && w.J.p && blu_LU<S>(s, false), "Autotune before Pack and NSPrepare");
             DevBuf<S> scratch;
             scratch.zero(n, st);
+            InCall one(s);
             auto pair_ms = [&] {
                 return time_ms(st, reps, [&] {
                     blusgs_sweep_into<S, EX>(s, false, false, w.rhs.p, scratch.p);
@@ -1158,7 +1204,7 @@ ucfd_status_t UCFDLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal turb_factor, UCFD
         // other into the same arrays, each with its own scattered pass).  Below
         // this size the scattered writes stay in L2 and one pass is faster.
         // (Not into a graph, whose every launch would write the same stamp.)
-        if (s->nelem == 1 && s->N >= kPackRecords && !capturing(s)) {
+        if (s->nelem == 1 && s->N >= kPackRecords && capture_id(s) == 0) {
             const bool fresh = w.rec.p == nullptr;
             S *rec = w.rec.ensure((size_t)kfast::pack_record_words<S>(s->nvars) * s->N);
             if (fresh) w.rec.zero(w.rec.n, st);  // no stamp from whatever was there
@@ -1344,6 +1390,7 @@ ucfd_status_t UCFDBLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal a0) {
     dispatch(s, [&]<typename S, bool EX>() {
         blusgs_alloc<S>(s);
         double *r64 = std::is_same<S, float>::value ? s->rhs64.p : nullptr;
+        block_capture_id(s);
         KCALL(EX, fs_blusgs_pack<S>, e.neles, s->nvars, s->nfvars, s->N, a0, ids, s->d_iperm.p, rh, dt,
               blu_rhs<S>(s), r64, s->dd.p, st);
     });
@@ -1369,6 +1416,7 @@ static ucfd_status_t tpack_api(FlowSys s, int model, UCFDInt eidx, UCFDReal fact
     const double *ds = device_view<double>(e.dsrc, nv, e.s_dsrc, st);
     const double *dt = device_view<double>(e.dt, e.neles, e.s_dt, st);
     dispatch(s, [&]<typename S, bool EX>() { blusgs_alloc<S>(s); });
+    block_capture_id(s);
     kfast::fs_tblusgs_pack(model, e.neles, s->nvars, s->ntvars, s->N, a0, factor, constants().betast, ids,
                            s->d_iperm.p, up, ds, dt, s->tD.p, st);
     s->c_valid[1] = false;
@@ -1412,6 +1460,7 @@ static ucfd_status_t blusgs_prepare_api(FlowSys s, bool turb) {
             if (!turb) J64 = s->J64.ensure(tiled_size(s->N, (long long)s->P * B * B));
         }
         double *jt = s->jt.ensure((size_t)2 * B * B * s->nfaces);
+        block_capture_id(s);
         KCALL(EX, fs_blusgs_prepare<S>, B, s->N, s->P, (long long)s->nfaces, s->d_nei.p, s->d_slot.p, s->d_side.p,
               s->fa64.p, s->rv64.p, jd, dd, D, LU64, LU_s, turb ? w.tJ.p : w.J.p, J64, jt, st);
     });
@@ -1435,8 +1484,12 @@ static ucfd_status_t blusgs_sweep_api(FlowSys s, bool turb, bool upper) {
         UCFD_REQUIRE(blu_LU<S>(s, turb), "sweep before Prepare");
         blusgs_sweep_into<S, EX>(s, turb, upper, sweep_rhs<S, EX>(s, turb), w.bdu.p);
     });
-    s->du64_valid = false;
-    s->x_zero = false;
+    if (capture_id(s) == 0) {
+        s->du64_valid = false;
+        s->x_zero = false;
+    } else if (s->prec == UCFD_PREC_FP32) {
+        UCFD_CUDA(cudaMemsetAsync(s->d_du_newer.p, 1, sizeof(int), s->stream()));
+    }
     finish(s);
     if (!s->async) check_sweep_err(s);
     UCFD_API_END
@@ -1466,8 +1519,10 @@ ucfd_status_t UCFDBLUSGS_Reset(FlowSys s) {
             split_forget(s);  // the next sweep forms every term of the zero increments itself
         }
     });
-    s->du64_valid = false;
-    s->x_zero = true;
+    if (block_capture_id(s) == 0) {  // (captured: du and x64 are both zero when it has run)
+        s->du64_valid = false;
+        s->x_zero = true;
+    }
     finish(s);
     UCFD_API_END
 }
@@ -1506,6 +1561,7 @@ ucfd_status_t UCFDBLUSGS_Update(FlowSys s, UCFDInt eidx) {
     const bool dev = is_device_ptr(e.uptsb);
     double *up = dev ? e.uptsb : const_cast<double *>(device_view<double>(e.uptsb, nv, e.s_upts, st));
     if (s->prec == UCFD_PREC_FP32 && s->du64_valid) {
+        x64_from_du(s);
         kfast::fs_blusgs_update<double>(e.neles, s->nvars, s->N, ids, s->d_iperm.p, s->x64.p, up, st);
     } else {
         dispatch(s, [&]<typename S, bool EX>() {
@@ -1527,13 +1583,14 @@ ucfd_status_t UCFDBLUSGS_Residual(FlowSys s, UCFDReal *relres) {
     double rn = 0, bn = 0;
     if (s->prec == UCFD_PREC_FP32) {
         UCFD_REQUIRE(s->J64.p, "Residual before NSPrepare");
+        x64_from_du(s);
         if (s->du64_valid)
-            blusgs_residual<double, double, false>(s, s->x_zero ? nullptr : s->x64.p, (double *)nullptr, &rn, &bn);
+            blusgs_residual<double, double, false>(s, x_is_zero(s) ? nullptr : s->x64.p, (double *)nullptr, &rn, &bn);
         else
-            blusgs_residual<float, float, false>(s, s->x_zero ? nullptr : s->w32.bdu.p, (float *)nullptr, &rn, &bn);
+            blusgs_residual<float, float, false>(s, x_is_zero(s) ? nullptr : s->w32.bdu.p, (float *)nullptr, &rn, &bn);
     } else {
         UCFD_REQUIRE(s->w64.J.p, "Residual before NSPrepare");
-        blusgs_residual<double, double, false>(s, s->x_zero ? nullptr : s->w64.bdu.p, (double *)nullptr, &rn, &bn);
+        blusgs_residual<double, double, false>(s, x_is_zero(s) ? nullptr : s->w64.bdu.p, (double *)nullptr, &rn, &bn);
     }
     *relres = bn > 0 ? rn / bn : rn;
     UCFD_API_END
@@ -1548,6 +1605,7 @@ ucfd_status_t UCFDBLUSGS_Solve(FlowSys s, UCFDReal rtol, UCFDInt max_sweeps, UCF
     cudaStream_t st = s->stream();
     int pairs = 0;
     double rn = 0, bn = 0, rel = 0;
+    InCall one(s);
     if (s->prec == UCFD_PREC_FP32) {
         Work<float> &w = s->w32;
         UCFD_REQUIRE(s->J64.p && w.LU.p, "Solve before NSPrepare");
@@ -1555,7 +1613,8 @@ ucfd_status_t UCFDBLUSGS_Solve(FlowSys s, UCFDReal rtol, UCFDInt max_sweeps, UCF
         w.r.ensure(n);
         w.delta.ensure(n);
         if (!s->du64_valid) kfast::convert<float, double>((long long)n, w.bdu.p, s->x64.p, st);
-        blusgs_residual<double, float, false>(s, s->x_zero ? nullptr : s->x64.p, w.r.p, &rn, &bn);
+        else x64_from_du(s);
+        blusgs_residual<double, float, false>(s, x_is_zero(s) ? nullptr : s->x64.p, w.r.p, &rn, &bn);
         rel = bn > 0 ? rn / bn : rn;
         while (rel > rtol && pairs < max_sweeps) {
             // the sweeps' right-hand side D^-1 r (their blocks are D^-1 J fv)
@@ -1576,12 +1635,13 @@ ucfd_status_t UCFDBLUSGS_Solve(FlowSys s, UCFDReal rtol, UCFDInt max_sweeps, UCF
         }
         kfast::convert<double, float>((long long)n, s->x64.p, w.bdu.p, st);
         s->du64_valid = true;
+        if (s->captured) s->d_du_newer.zero(1, st);
         split_forget(s);  // du now holds the refined solution
     } else {
         Work<double> &w = s->w64;
         UCFD_REQUIRE(w.J.p, "Solve before NSPrepare");
         const bool ex = s->prec == UCFD_PREC_FP64;
-        blusgs_residual<double, double, false>(s, s->x_zero ? nullptr : w.bdu.p, (double *)nullptr, &rn, &bn);
+        blusgs_residual<double, double, false>(s, x_is_zero(s) ? nullptr : w.bdu.p, (double *)nullptr, &rn, &bn);
         rel = bn > 0 ? rn / bn : rn;
         while (rel > rtol && pairs < max_sweeps) {
             const int m = std::min(inner_sweeps, max_sweeps - pairs);
@@ -1640,4 +1700,8 @@ bool ucfd::flowsys_block_view(FlowSys s, BlockSystemView &v) {
     t.stream = (void *)s->stream();
     v = t;
     return true;
+}
+
+void ucfd::flowsys_block_view_refresh(FlowSys s) {
+    if (s->prec == UCFD_PREC_FP32) x64_from_du(s);
 }

@@ -22,5 +22,8 @@ struct BlockSystemView {
 // Fills v for a FlowSys whose BLU-SGS system has been packed and prepared;
 // returns false (and leaves v untouched) otherwise.  Never allocates.
 bool flowsys_block_view(FlowSys s, BlockSystemView &v);
+// Enqueues on the view's stream what brings its x up to date (nothing, unless
+// block sweeps were captured into a graph).  The handle's device is current.
+void flowsys_block_view_refresh(FlowSys s);
 
 }  // namespace ucfd

@@ -123,6 +123,7 @@
     void fingerprint(long long n, const int *a, unsigned long long *out, cudaStream_t s);          \
     template <typename Ts, typename Td>                                                            \
     void convert(long long n, const Ts *src, Td *dst, cudaStream_t s);                             \
+    void widen_if(long long n, const int *flag, const float *src, double *dst, cudaStream_t s);    \
     template <typename Ts>                                                                         \
     void axpy_into(long long n, const Ts *x, double *y, cudaStream_t s);                           \
     template <typename S>                                                                          \

@@ -784,6 +784,17 @@ void convert(long long n, const Ts *src, Td *dst, cudaStream_t s) {
     convert_kernel<Ts, Td><<<grid_for(n < (1ll << 24) ? n : (1ll << 24)), kBlock, 0, s>>>(n, src, dst);
 }
 
+// dst = src where *flag is set.
+__global__ void widen_if_kernel(long long n, const int *flag, const float *src, double *dst) {
+    if (*flag == 0) return;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        dst[i] = to_double(src[i]);
+}
+
+void widen_if(long long n, const int *flag, const float *src, double *dst, cudaStream_t s) {
+    if (n > 0) widen_if_kernel<<<vec_grid(n), kBlock, 0, s>>>(n, flag, src, dst);
+}
+
 template <typename Ts>
 __global__ void axpy_into_kernel(long long n, const Ts *x, double *y) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)

@@ -210,6 +210,7 @@ extern "C" ucfd_status_t UCFDBLUSGS_ResidualNoAlloc(FlowSys sys, UCFDReal *relre
     double *scratch = g_scratch_addr[dev].load(std::memory_order_acquire);
     cudaStream_t s = (cudaStream_t)v.stream;
     const int nb = (int)((v.N + kCellsPerBlock - 1) / kCellsPerBlock);
+    ucfd::flowsys_block_view_refresh(sys);
     if (v.x64) launch<double>(v, v.x64, scratch, nb, s);
     else launch<float>(v, v.x32, scratch, nb, s);
     const bool out_dev = ucfd::is_device_ptr(relres);
