@@ -104,6 +104,7 @@ struct _FlowSys {
     // state (split, c_valid, x_zero) holds within one capture, in the order of
     // the graph, and within one call (in_call), and no longer.
     bool captured = false;
+    bool captured_inputs = false;  // among them a Pack or Prepare: what sweeps start from may change too
     bool in_call = false;
     bool bulk_captured = false;  // ... with a bulk-copy variant
     bool du64_valid = false;
@@ -539,10 +540,17 @@ unsigned long long block_capture_id(FlowSys s) {
     return id;
 }
 
+// The same for a Pack or Prepare.
+unsigned long long input_capture_id(FlowSys s) {
+    const unsigned long long id = block_capture_id(s);
+    s->captured_inputs = s->captured_inputs || id != 0;
+    return id;
+}
+
 // Whether what a call under capture `then` left on the device is still there
-// for a call under capture `now`.
-bool still_holds(FlowSys s, unsigned long long then, unsigned long long now) {
-    return then == now && (now != 0 || !s->captured || s->in_call);
+// for a call under capture `now`; graphs: some may run in between.
+bool still_holds(FlowSys s, unsigned long long then, unsigned long long now, bool graphs) {
+    return then == now && (now != 0 || !graphs || s->in_call);
 }
 
 // Right-hand side of the fast modes' block sweeps (their blocks are
@@ -556,7 +564,7 @@ const S *sweep_rhs(FlowSys s, bool turb) {
     const int B = turb ? s->ntvars : s->nfvars;
     const int var0 = turb ? s->nfvars : 0;
     const unsigned long long now = block_capture_id(s);
-    if (!s->c_valid[turb ? 1 : 0] || !still_holds(s, s->c_capture[turb ? 1 : 0], now)) {
+    if (!s->c_valid[turb ? 1 : 0] || !still_holds(s, s->c_capture[turb ? 1 : 0], now, s->captured_inputs)) {
         w.crhs.ensure((size_t)s->nvars * s->N);
         kfast::fs_blusgs_rhs_solve<S>(B, s->N, var0, blu_LU<S>(s, turb), w.rhs.p, w.crhs.p, s->stream());
         s->c_valid[turb ? 1 : 0] = true;
@@ -583,7 +591,7 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     sp.nvars = s->nvars;
     const unsigned long long now = block_capture_id(s);
     sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0] &&
-               still_holds(s, ss.capture, now)) ? 0 : 1;
+               still_holds(s, ss.capture, now, s->captured)) ? 0 : 1;
     const S *fa = geo_fa<S>(s);
     if constexpr (EX) fa = s->fv64.p;
     if (s->variant == 2 || s->variant == 3) {
@@ -628,10 +636,8 @@ void split_forget(FlowSys s) { s->split[0] = s->split[1] = SplitState{}; }
 struct InCall {
     FlowSys s;
     explicit InCall(FlowSys h) : s(h) {
-        if (s->captured) {
-            split_forget(s);
-            s->c_valid[0] = s->c_valid[1] = false;
-        }
+        if (s->captured) split_forget(s);
+        if (s->captured_inputs) s->c_valid[0] = s->c_valid[1] = false;
         s->in_call = true;
     }
     ~InCall() { s->in_call = false; }
@@ -1390,7 +1396,7 @@ ucfd_status_t UCFDBLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal a0) {
     dispatch(s, [&]<typename S, bool EX>() {
         blusgs_alloc<S>(s);
         double *r64 = std::is_same<S, float>::value ? s->rhs64.p : nullptr;
-        block_capture_id(s);
+        input_capture_id(s);
         KCALL(EX, fs_blusgs_pack<S>, e.neles, s->nvars, s->nfvars, s->N, a0, ids, s->d_iperm.p, rh, dt,
               blu_rhs<S>(s), r64, s->dd.p, st);
     });
@@ -1416,7 +1422,7 @@ static ucfd_status_t tpack_api(FlowSys s, int model, UCFDInt eidx, UCFDReal fact
     const double *ds = device_view<double>(e.dsrc, nv, e.s_dsrc, st);
     const double *dt = device_view<double>(e.dt, e.neles, e.s_dt, st);
     dispatch(s, [&]<typename S, bool EX>() { blusgs_alloc<S>(s); });
-    block_capture_id(s);
+    input_capture_id(s);
     kfast::fs_tblusgs_pack(model, e.neles, s->nvars, s->ntvars, s->N, a0, factor, constants().betast, ids,
                            s->d_iperm.p, up, ds, dt, s->tD.p, st);
     s->c_valid[1] = false;
@@ -1460,7 +1466,7 @@ static ucfd_status_t blusgs_prepare_api(FlowSys s, bool turb) {
             if (!turb) J64 = s->J64.ensure(tiled_size(s->N, (long long)s->P * B * B));
         }
         double *jt = s->jt.ensure((size_t)2 * B * B * s->nfaces);
-        block_capture_id(s);
+        input_capture_id(s);
         KCALL(EX, fs_blusgs_prepare<S>, B, s->N, s->P, (long long)s->nfaces, s->d_nei.p, s->d_slot.p, s->d_side.p,
               s->fa64.p, s->rv64.p, jd, dd, D, LU64, LU_s, turb ? w.tJ.p : w.J.p, J64, jt, st);
     });
