@@ -111,6 +111,10 @@ UCFD_EXTERN ucfd_status_t UCFDDeviceInfo(char *name, size_t len, int *sm_count);
  * whether each gave up as designed (1) -- instead of hanging -- leaving the
  * context usable.  No counterpart in the reference. */
 UCFD_EXTERN ucfd_status_t UCFDSelfTestTimeouts(int *barrier_timed_out, int *mbarrier_timed_out);
+/* Memory that calls are faster with and can do without, in pieces of more than
+ * `bytes`, counts as not to be had in calls of this thread (0: no limit): the
+ * forms that do without it can be tested with memory to spare. */
+UCFD_EXTERN ucfd_status_t UCFDSelfTestScratchLimit(size_t bytes);
 
 #if defined(__cplusplus)
 }

@@ -586,10 +586,16 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     // sweep in full mode)
     SweepSplit<S> sp;
     SplitState &ss = s->split[turb ? 1 : 0];
-    sp.part = w.spart.ensure((size_t)(EX ? s->P : 1) * s->nvars * s->N);
+    const unsigned long long now = block_capture_id(s);
+    if constexpr (EX) {
+        // nullptr (no room, or no sweep would read them): the terms are not kept
+        sp.part = !s->has_self && still_holds(s, now, now, s->captured) ? w.spart.p : nullptr;
+        if (!sp.part) ss = SplitState{};
+    } else {
+        sp.part = w.spart.ensure((size_t)s->nvars * s->N);
+    }
     sp.upper = upper ? 1 : 0;
     sp.nvars = s->nvars;
-    const unsigned long long now = block_capture_id(s);
     sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0] &&
                still_holds(s, ss.capture, now, s->captured)) ? 0 : 1;
     const S *fa = geo_fa<S>(s);
@@ -615,7 +621,7 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
               s->block, s->variant, s->d_sweep_err.p, kBulkMaxSpin, sp, s->stream());
         if (s->sch.lev_off[l + 1] > s->sch.lev_off[l]) sp.chained = 1;
     }
-    ss = SplitState{du, upper ? 1 : 0, s->jver[turb ? 1 : 0], rhs, s->rver, now};
+    if (sp.part) ss = SplitState{du, upper ? 1 : 0, s->jver[turb ? 1 : 0], rhs, s->rver, now};
 }
 
 // du of the fast block sweeps was set to zero: both sides' sums are zero,
@@ -1466,7 +1472,15 @@ static ucfd_status_t blusgs_prepare_api(FlowSys s, bool turb) {
             if (!turb) J64 = s->J64.ensure(tiled_size(s->N, (long long)s->P * B * B));
         }
         double *jt = s->jt.ensure((size_t)2 * B * B * s->nfaces);
-        input_capture_id(s);
+        // What the sweeps keep, allocated here so that the first of them can be
+        // captured: the exact mode's terms (P nvars doubles a cell, 240 bytes
+        // for a hexahedron's six faces and five variables) where there is room
+        // and no face leads to the cell itself; the other modes' sums and
+        // right-hand sides, without which a sweep would fail
+        if (input_capture_id(s) == 0 && (!EX || !s->has_self)) {
+            w.spart.try_ensure((size_t)(EX ? s->P : 1) * s->nvars * s->N);
+            if (!EX) w.crhs.try_ensure((size_t)s->nvars * s->N);
+        }
         KCALL(EX, fs_blusgs_prepare<S>, B, s->N, s->P, (long long)s->nfaces, s->d_nei.p, s->d_slot.p, s->d_side.p,
               s->fa64.p, s->rv64.p, jd, dd, D, LU64, LU_s, turb ? w.tJ.p : w.J.p, J64, jt, st);
     });

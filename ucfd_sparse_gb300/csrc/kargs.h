@@ -87,7 +87,8 @@ struct ScalarSweepArgs {
 //   Fast build (M = D^-1 J fv blocks): one sum per side, S_lo and S_up, and
 //     du = c - S_lo - S_up; part [nvars][N].
 //   Exact build: the reference subtracts the faces one by one in face order,
-//     so each face's rounded term is kept; part [P][nvars][N].
+//     so each face's rounded term is kept; part [P][nvars][N], or nullptr
+//     where no later sweep would read it (then full == 1).
 // (A face to the cell itself is formed by every sweep; a mesh with such
 // faces always sweeps in full mode.)
 template <typename S>

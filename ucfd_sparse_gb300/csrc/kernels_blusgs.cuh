@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, lo
             for (int c = 1; c < B; ++c) val += __ldcs(Jp + ((r * B + c) << 5)) * x[c];
             val *= fv;
             b[r] -= val;
-            if (sd == sp.upper) term[r * N] = val;
+            if (sd == sp.upper && sp.part) term[r * N] = val;
         }
     };
     if constexpr (PW > 0) {
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(32) fs_blusgs_sweep_rows_kernel(int t0, int t1
             for (int q = 1; q < B; ++q) val += jv[p][q] * x[p][q];
             val *= f[p];
             b -= val;
-            if (valid && (own >> p) & 1u) sp.part[((long long)p * sp.nvars + var0 + r) * N + k] = val;
+            if (valid && sp.part && (own >> p) & 1u) sp.part[((long long)p * sp.nvars + var0 + r) * N + k] = val;
         } else if (nb[p] >= 0) {
             b -= kept[p];
         }

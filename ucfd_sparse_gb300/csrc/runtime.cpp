@@ -100,7 +100,10 @@ int sm_count() {
 
 namespace {
 std::atomic<int> g_host_access{UCFD_HOST_MAP};
+thread_local size_t g_scratch_limit = SIZE_MAX;
 }
+
+size_t &scratch_limit() { return g_scratch_limit; }
 
 const void *host_mapped(const void *ptr) {
     if (!ptr || g_host_access.load(std::memory_order_relaxed) != UCFD_HOST_MAP) return nullptr;
@@ -171,6 +174,12 @@ ucfd_status_t UCFDGetTransferStats(UCFDTransferStats *stats) {
 }
 
 const char *UCFDVersion(void) { return "ucfd_gb300 1.0 (sm_103a)"; }
+
+ucfd_status_t UCFDSelfTestScratchLimit(size_t bytes) {
+    UCFD_API_BEGIN
+    ucfd::scratch_limit() = bytes ? bytes : SIZE_MAX;
+    UCFD_API_END
+}
 
 ucfd_status_t UCFDDeviceInfo(char *name, size_t len, int *sm) {
     UCFD_API_BEGIN

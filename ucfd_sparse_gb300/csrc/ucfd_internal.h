@@ -55,6 +55,10 @@ inline void cuda_check(cudaError_t e, const char *what, const char *file, int li
 void copy_h2d(void *dst, const void *src, size_t bytes, cudaStream_t s);
 void copy_d2h(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
+// Largest allocation (bytes) that DevBuf::try_ensure makes on this thread:
+// no limit, unless UCFDSelfTestScratchLimit has one stand for full memory.
+size_t &scratch_limit();
+
 template <typename T>
 struct DevBuf {
     T *p = nullptr;
@@ -91,6 +95,20 @@ struct DevBuf {
             p = nullptr;
             cudaGetLastError();
             fail(UCFD_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+        }
+        n = count;
+        return p;
+    }
+    // Memory that a call is faster with and can do without: nullptr where
+    // there is not as much.
+    T *try_ensure(size_t count) {
+        if (count <= n && p) return p;
+        release();
+        const size_t bytes = (count ? count : 1) * sizeof(T);
+        if (bytes > scratch_limit() || cudaMalloc((void **)&p, bytes) != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();
+            return nullptr;
         }
         n = count;
         return p;

@@ -74,6 +74,7 @@ SIGNATURES = {
     "UCFDVersion": (c_char_p, []),
     "UCFDDeviceInfo": (_I, [c_char_p, c_size_t, POINTER(c_int)]),
     "UCFDSelfTestTimeouts": (_I, [POINTER(c_int), POINTER(c_int)]),
+    "UCFDSelfTestScratchLimit": (_I, [c_size_t]),
     "UCFDSetTransferTiming": (_I, [_I]),
     "UCFDGetTransferStats": (_I, [_P]),
     "UCFDSetHostArrayAccess": (_I, [_I]),
