@@ -151,6 +151,8 @@ constexpr int kActLevel = 16384;
 // Cells from which Pack goes through records.
 constexpr long long kPackRecords = 131072;
 
+void pack_records_alloc(FlowSys s);
+
 // Build the level schedule and the ELL mesh arrays (once).
 void build_topology(FlowSys s) {
     if (s->topo) return;
@@ -258,6 +260,7 @@ void build_topology(FlowSys s) {
         std::vector<float> h(enrm.begin(), enrm.end());
         s->w32.nrm.upload(h.data(), h.size(), st);
     }
+    pack_records_alloc(s);
     UCFD_CUDA(cudaStreamSynchronize(st));
     s->topo = true;
 }
@@ -464,6 +467,18 @@ void lusgs_alloc(FlowSys s) {
     w.diag.ensure(n);
     w.base.ensure(n);
     w.rhs0.ensure(n);
+}
+
+// Pack's records (112 bytes a cell for six variables in FP32), allocated with
+// the schedule, beside whose host work that takes no time, so that no Pack pays
+// for it; where there is no room Pack goes without.
+void pack_records_alloc(FlowSys s) {
+    if (s->nelem != 1 || s->N < kPackRecords || s->mode == MODE_BLUSGS || s->nvars < 4 || s->nvars > 7) return;
+    dispatch(s, [&]<typename S, bool EX>() {
+        DevBuf<S> &rec = work<S>(s).rec;
+        const size_t n = (size_t)kfast::pack_record_words<S>(s->nvars) * s->N;
+        if (rec.try_ensure(n)) rec.zero(n, s->stream());  // no stamp from whatever was there
+    });
 }
 
 // ---- block LU-SGS -----------------------------------------------------------
@@ -1212,14 +1227,13 @@ ucfd_status_t UCFDLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal turb_factor, UCFD
         lusgs_alloc<S>(s);
         Work<S> &w = work<S>(s);
         if constexpr (std::is_same<S, float>::value) w.ulo.ensure((size_t)s->nvars * s->N);
-        // one element: through records (several elements pack one after the
-        // other into the same arrays, each with its own scattered pass).  Below
-        // this size the scattered writes stay in L2 and one pass is faster.
+        // one element of all cells: through records (several elements pack one
+        // after the other into the same arrays, each with its own scattered
+        // pass).  Below kPackRecords cells, where no records are allocated, the
+        // scattered writes stay in L2 and one pass is faster.
         // (Not into a graph, whose every launch would write the same stamp.)
-        if (s->nelem == 1 && s->N >= kPackRecords && capture_id(s) == 0) {
-            const bool fresh = w.rec.p == nullptr;
-            S *rec = w.rec.ensure((size_t)kfast::pack_record_words<S>(s->nvars) * s->N);
-            if (fresh) w.rec.zero(w.rec.n, st);  // no stamp from whatever was there
+        S *rec = w.rec.p;
+        if (rec && e.neles == s->N && capture_id(s) == 0) {
             if (++s->pack_stamp <= 0) s->pack_stamp = 1;
             bool ok = false;
             if constexpr (EX)
@@ -1383,6 +1397,8 @@ ucfd_status_t UCFDFlowSysSetBLUSGS(FlowSys *sys, UCFDReal *jmat, UCFDReal *tjmat
     FlowSys s = *sys;
     UCFD_REQUIRE(s->mode == MODE_NONE || s->mode == MODE_BLUSGS, "FlowSys already set up for LU-SGS");
     s->mode = MODE_BLUSGS;
+    s->w64.rec.release();
+    s->w32.rec.release();
     s->jmat = jmat;
     s->tjmat = tjmat;
     UCFD_API_END
