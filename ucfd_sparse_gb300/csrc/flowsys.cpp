@@ -765,19 +765,16 @@ void run_graph_drop(FlowSys s) {
 }
 
 // FP32 sweeps of both systems: the packed per cell-face geometry (fixed with
-// the mesh) and room for both spectral radii; nullptr in FP64.
+// the mesh).  Its first call comes after the launches that do not read it: the
+// allocation then takes place beside them.
 template <typename S>
-void *pack_geo(FlowSys s, cudaStream_t st) {
+void pack_geo(FlowSys s, cudaStream_t st) {
     if constexpr (std::is_same<S, float>::value) {
         Work<S> &w = work<S>(s);
-        const long long nl = (long long)s->P * s->N;
-        if (!w.geo4.p) {
-            w.geo4.ensure((size_t)nl);
-            kfast::pack_geo4(s->N, s->P, s->ndims, w.nrm.p, geo_fa<S>(s), geo_rv<S>(s), w.geo4.p, st);
-        }
-        return w.lam2.ensure((size_t)nl);
+        if (w.geo4.p) return;
+        w.geo4.ensure((size_t)s->P * s->N);
+        kfast::pack_geo4(s->N, s->P, s->ndims, w.nrm.p, geo_fa<S>(s), geo_rv<S>(s), w.geo4.p, st);
     }
-    return nullptr;
 }
 
 // And both spectral radii, from lamN and lamT as just gathered.
@@ -785,7 +782,9 @@ template <typename S>
 void pack_both(FlowSys s, cudaStream_t st) {
     if constexpr (std::is_same<S, float>::value) {
         Work<S> &w = work<S>(s);
-        kfast::pack_lam2((long long)s->P * s->N, w.lamN.p, w.lamT.p, pack_geo<S>(s, st), st);
+        const long long nl = (long long)s->P * s->N;
+        kfast::pack_lam2(nl, w.lamN.p, w.lamT.p, w.lam2.ensure((size_t)nl), st);
+        pack_geo<S>(s, st);
         s->lam2_ok = true;
     }
 }
@@ -1311,11 +1310,12 @@ static ucfd_status_t lusgs_prepare_api(FlowSys s, int sys, UCFDReal kappa) {
         if (lfT) w.lamT.ensure((size_t)nl);
         s->lam2_ok = false;
         void *lam2 = nullptr;
-        if (sys == 2) lam2 = pack_geo<S>(s, st);
+        if (sys == 2 && std::is_same<S, float>::value) lam2 = w.lam2.ensure((size_t)nl);
         KCALL(EX, fs_lusgs_gather_prepare<S>, s->N, s->P, sys == 1 ? s->nfvars : 0, s->nfvars,
               sys == 0 ? s->nfvars : s->nvars, (S)kappa, s->d_slot.p, geo_fa<S>(s), geo_rv<S>(s),
               sys == 1 ? lfT : lfN, sys == 2 ? lfT : nullptr, sys == 1 ? w.lamT.p : w.lamN.p, w.lamT.p, lam2,
               w.diag.p, st);
+        if (lam2) pack_geo<S>(s, st);
         s->lam2_ok = lam2 != nullptr;
     });
     finish(s, (lfN && !is_device_ptr(s->fspr)) || (lfT && !is_device_ptr(s->tfspr)));
