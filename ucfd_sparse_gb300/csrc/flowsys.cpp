@@ -452,10 +452,10 @@ void lusgs_sweep(FlowSys s, int sys, bool upper, double kappa, bool persistent =
 }
 
 template <typename S, bool EX>
-void lusgs_prepare(FlowSys s, bool rans, double kappa, const S *base) {
+void lusgs_prepare(FlowSys s, bool rans, double kappa) {
     Work<S> &w = work<S>(s);
     KCALL(EX, fs_lusgs_prepare<S>, s->N, s->P, rans ? s->nfvars : 0, rans ? s->nvars : s->nfvars, (S)kappa,
-          s->d_nei.p, geo_fa<S>(s), geo_rv<S>(s), rans ? w.lamT.p : w.lamN.p, base, w.diag.p, s->stream());
+          s->d_nei.p, geo_fa<S>(s), geo_rv<S>(s), rans ? w.lamT.p : w.lamN.p, w.base.p, w.diag.p, s->stream());
 }
 
 template <typename S>
@@ -725,8 +725,8 @@ void lusgs_run_prepare(FlowSys s, bool rans, double kappa, bool persistent) {
         KCALL(EX, fs_lusgs_prepare_both<S>, s->N, s->P, s->nfvars, s->nvars, (S)kappa, s->d_nei.p, geo_fa<S>(s),
               geo_rv<S>(s), w.lamN.p, w.lamT.p, w.base.p, w.diag.p, s->stream());
     } else {
-        lusgs_prepare<S, EX>(s, false, kappa, w.base.p);
-        if (rans) lusgs_prepare<S, EX>(s, true, kappa, w.base.p);
+        lusgs_prepare<S, EX>(s, false, kappa);
+        if (rans) lusgs_prepare<S, EX>(s, true, kappa);
     }
 }
 

@@ -328,65 +328,38 @@ __global__ void __launch_bounds__(256) pc_upper_kernel(int t0, int t1, int bn, i
     }
 }
 
-// One level of the ILU(0) factorisation in place on the caller's BSR
-// values (row-major B x B blocks in CSR slot order), one thread per row
-// (rows[t] for t in [t0, t1), every lower neighbour already final):
-// precon/bilu.c:5-62 (SCALAR false) or precon/ilu.c:4-47 (SCALAR, B = 1).
-// For each lower slot k of row i in order: A_ik := A_ik inv(A_kk)
-// (lusubmattrans; A_ik / a_kk when SCALAR), then A_ij -= A_ik A_kj for
-// every later slot j whose column row k holds (the last such slot of row k,
-// as the reference's column map keeps); finally the diagonal block is
-// LU-factorised (block ILU only).
-template <int B, bool SCALAR>
-__global__ void ilu_factor_kernel(int t0, int t1, const int *rows, const int *rowptr, const int *colidx,
-                                  const int *diagslots, double *vals) {
+// One level of the ILU(0) factorisation in place on the caller's BSR values
+// (row-major B x B blocks in CSR slot order; rows[t] for t in [t0, t1), every
+// lower neighbour already final): precon/bilu.c:5-62 or, for scalar ILU,
+// precon/ilu.c:4-47.  For each lower slot k of row i in order: A_ik := A_ik
+// inv(A_kk) (A_ik / a_kk for scalar ILU), then A_ij -= A_ik A_kj for every
+// later slot j whose column row k holds (the last such slot of row k, as the
+// reference's column map keeps); finally the diagonal block is LU-factorised
+// (block ILU only).
+//
+// Blocks of one value, one thread per row.  SCALAR: ILU(0); otherwise block
+// ILU of block size 1, whose factored diagonal is the reciprocal pivot.
+template <bool SCALAR>
+__global__ void ilu_factor_scalar_kernel(int t0, int t1, const int *rows, const int *rowptr, const int *colidx,
+                                         const int *diagslots, double *vals) {
     const int t = t0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= t1) return;
-    constexpr int B2 = B * B;
     const int i = rows ? rows[t] : t;
     const int st = rowptr[i], ed = diagslots[i], jed = rowptr[i + 1];
     for (int kd = st; kd < ed; ++kd) {
-        const int ck = colidx[kd], kk = diagslots[ck], kst = rowptr[ck], ked = rowptr[ck + 1];
-        double aik[B2];
-#pragma unroll
-        for (int e = 0; e < B2; ++e) aik[e] = vals[(long long)kd * B2 + e];
-        if constexpr (SCALAR) {
-            aik[0] = aik[0] / vals[kk];
-        } else {
-            double lu[B2];
-#pragma unroll
-            for (int e = 0; e < B2; ++e) lu[e] = vals[(long long)kk * B2 + e];
-            lusubmattrans_dev<double, B>(lu, aik);
-        }
-#pragma unroll
-        for (int e = 0; e < B2; ++e) vals[(long long)kd * B2 + e] = aik[e];
+        const int ck = colidx[kd], kst = rowptr[ck], ked = rowptr[ck + 1];
+        const double akk = vals[diagslots[ck]];
+        const double aik = SCALAR ? vals[kd] / akk : vals[kd] * akk;
+        vals[kd] = aik;
         for (int jj = kd + 1; jj < jed; ++jj) {
             const int cj = colidx[jj];
             int iwj = -1;
             for (int q = kst; q < ked; ++q)
                 if (colidx[q] == cj) iwj = q;
-            if (iwj < 0) continue;
-            const double *akj = vals + (long long)iwj * B2;
-            double *aij = vals + (long long)jj * B2;
-#pragma unroll
-            for (int r = 0; r < B; ++r)
-#pragma unroll
-                for (int c = 0; c < B; ++c) {
-                    double v = 0.0;
-#pragma unroll
-                    for (int e = 0; e < B; ++e) v += aik[r * B + e] * akj[e * B + c];
-                    aij[r * B + c] -= v;
-                }
+            if (iwj >= 0) vals[jj] -= mul_rn(aik, vals[iwj]);
         }
     }
-    if constexpr (!SCALAR) {
-        double d[B2];
-#pragma unroll
-        for (int e = 0; e < B2; ++e) d[e] = vals[(long long)ed * B2 + e];
-        ludcmp_dev<double, B>(d);
-#pragma unroll
-        for (int e = 0; e < B2; ++e) vals[(long long)ed * B2 + e] = d[e];
-    }
+    if (!SCALAR) vals[ed] = 1.0 / vals[ed];
 }
 
 // The block factorisation of one level with B lanes per row (32 / B rows per
@@ -420,7 +393,7 @@ __global__ void __launch_bounds__(32) ilu_factor_rows_kernel(int t0, int t1, con
             double x[B];
 #pragma unroll
             for (int e = 0; e < B; ++e) x[e] = own[e];
-            // row r of A_ik inv(LU): lusubmattrans_dev
+            // row r of X inv(LU) (lusubmattrans: src/krylov/utils/inverse.c:79-108): Y U = X, then X L = Y
             x[0] /= lu[0];
 #pragma unroll
             for (int row = 1; row < B; ++row) {

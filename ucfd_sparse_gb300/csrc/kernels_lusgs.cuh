@@ -817,10 +817,12 @@ __device__ __forceinline__ void scalar_sweep_lanes(const ScalarSweepArgs<double>
 
 // SYS: 0 mean flow, 1 turbulence, 2 both (blockIdx.y picks the system).  a.lam
 // is the system's spectral radius; with SYS == 2 tlam is the turbulence one.
+constexpr int kLanesThreads = 32;
+
 template <int NV, int NFV, int NDIMS, int SYS, int GF>
-__global__ void __launch_bounds__(64) scalar_sweep_lanes_kernel(ScalarSweepArgs<double> a) {
+__global__ void __launch_bounds__(kLanesThreads) scalar_sweep_lanes_kernel(ScalarSweepArgs<double> a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ double sm[64 / (2 * GF) * GF * NFV];
+    __shared__ double sm[kLanesThreads / 2 * NFV];
     if constexpr (SYS == 2) {
         if (blockIdx.y == 1) {
             a.lam = a.tlam;
@@ -1211,9 +1213,8 @@ __device__ __forceinline__ void prepare_sums(long long N, int maxdeg, long long 
     }
 }
 
-// pre_lusgs: lusgs.c:87-113.  lam is the per cell-face copy of lambdaf.
-// With base != nullptr the result is base + sd (a pseudo-time loop
-// re-preparing from the packed diagonal), otherwise diag += sd.
+// pre_lusgs: lusgs.c:87-113, for a pseudo-time loop: diag = base + sum, base
+// the packed diagonal, lam the per cell-face copy of lambdaf.
 template <typename T>
 __global__ void fs_lusgs_prepare_kernel(long long N, int maxdeg, int nv0, int nv1, T kappa,
                                         const int *nei, const T *fa, const T *rv, const T *lam,
@@ -1222,16 +1223,12 @@ __global__ void fs_lusgs_prepare_kernel(long long N, int maxdeg, int nv0, int nv
     if (k >= N) return;
     T sd, st;
     prepare_sums<T, false>(N, maxdeg, k, kappa, nei, fa, rv, lam, nullptr, sd, st);
-    if (base)
-        for (int v = nv0; v < nv1; ++v) diag[k + v * N] = base[k + v * N] + sd;
-    else
-        for (int v = nv0; v < nv1; ++v) diag[k + v * N] += sd;
+    for (int v = nv0; v < nv1; ++v) diag[k + v * N] = base[k + v * N] + sd;
 }
 
 // pre_lusgs of both systems in one pass over the faces: the mean-flow
 // variables [0, nfv) from lam, the turbulence variables [nfv, nv) from
-// tlam, each sum formed as fs_lusgs_prepare_kernel forms it;
-// diag = base + sum, or diag += sum without base.
+// tlam, each sum formed as fs_lusgs_prepare_kernel forms it.
 template <typename T>
 __global__ void fs_lusgs_prepare_both_kernel(long long N, int maxdeg, int nfv, int nv, T kappa, const int *nei,
                                              const T *fa, const T *rv, const T *lam, const T *tlam, const T *base,
@@ -1240,10 +1237,7 @@ __global__ void fs_lusgs_prepare_both_kernel(long long N, int maxdeg, int nfv, i
     if (k >= N) return;
     T sd, st;
     prepare_sums<T, true>(N, maxdeg, k, kappa, nei, fa, rv, lam, tlam, sd, st);
-    if (base)
-        for (int v = 0; v < nv; ++v) diag[k + v * N] = base[k + v * N] + (v < nfv ? sd : st);
-    else
-        for (int v = 0; v < nv; ++v) diag[k + v * N] += v < nfv ? sd : st;
+    for (int v = 0; v < nv; ++v) diag[k + v * N] = base[k + v * N] + (v < nfv ? sd : st);
 }
 
 // Prepare of a system (TWO: of both) straight from the face arrays: each cell

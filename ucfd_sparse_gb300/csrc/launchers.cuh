@@ -155,8 +155,8 @@ template <int NV, int NFV, int NDIMS, int SYS>
 static void sweep_lanes_go(const ::ucfd::ScalarSweepArgs<double> &a, int gf, cudaStream_t s) {
     const long long n = a.t1 - a.t0;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid_for(n * 2 * gf, 32), SYS == 2 ? 2 : 1);
-    cfg.blockDim = dim3(32);
+    cfg.gridDim = dim3(grid_for(n * 2 * gf, kLanesThreads), SYS == 2 ? 2 : 1);
+    cfg.blockDim = dim3(kLanesThreads);
     cfg.stream = s;
     // the next level's launch may start while this level runs
     cudaLaunchAttribute attr[1];
@@ -761,7 +761,7 @@ void ilu_factor(int B, int scalar, int t0, int t1, const int *rows, const int *r
     const unsigned g = grid_for(t1 - t0, block);
     if (scalar) {
         if (B != 1) ::ucfd::fail(UCFD_ERR_ARGUMENT, "scalar ILU needs block size 1 (got %d)", B);
-        ilu_factor_kernel<1, true><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
+        ilu_factor_scalar_kernel<true><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
         return;
     }
     if (B > 1) {
@@ -769,7 +769,7 @@ void ilu_factor(int B, int scalar, int t0, int t1, const int *rows, const int *r
                                                                                          diagslots, vals)));
         return;
     }
-    ilu_factor_kernel<1, false><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
+    ilu_factor_scalar_kernel<false><<<g, block, 0, s>>>(t0, t1, rows, rowptr, colidx, diagslots, vals);
 }
 
 template <typename Ts, typename Td>
