@@ -112,6 +112,12 @@ UCFD_EXTERN ucfd_status_t UCFDFlowSysSetLaunch(FlowSys sys, int threads_per_bloc
 
 /* Launch choices of the sweeps.  None of them changes any result: every
  * choice applies the same operations to each cell in the same order.
+ * Levels of some sizes have kernels with a launch shape of their own: FP64
+ * scalar levels with rows of at most eight faces, up to 8192 cells (6144 where
+ * a cell has more than four faces towards one side) and above 16384, take no
+ * notice of threads_per_block and have one kernel for sweep_variant 0, 1 and
+ * 2; FP64 block levels of up to 8192 cells with ELL width 4 or 6 have one for
+ * every choice.
  * No counterpart in the reference (its launch shape is the compile-time
  * TPB/BLOCK macro of Makefile.inc). */
 typedef struct {

@@ -86,3 +86,13 @@ def test_scalar_register_caps_of_fp64_levels(nvars, prec, port, ucfd):
                                       fs["fspr"], fs["tfspr"], kappa=1.01, a0=0.3, turb_factor=1.5,
                                       rans=nvars > 5)[0]
         np.testing.assert_array_equal(outs[0], ref)
+
+
+# colours of 8064 / 8065 (two lanes per face) and 8320 / 8321 quadrilaterals
+# (one thread per cell): either side of the line for rows of four faces
+@pytest.mark.parametrize("m", [127, 129])
+@pytest.mark.parametrize("nvars", [4, 6])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_plane_levels_either_side_of_the_lane_kernel(m, nvars, prec, ucfd):
+    from tests.test_gpu_level_shapes import test_plane_levels as same_as_two_threads_per_cell
+    same_as_two_threads_per_cell(m, nvars, prec, ucfd)

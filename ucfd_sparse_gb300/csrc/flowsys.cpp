@@ -144,11 +144,15 @@ void finish(FlowSys s, bool force_sync = false) {
     if (!s->async || force_sync) UCFD_CUDA(cudaStreamSynchronize(s->stream()));
 }
 
-// Largest level whose active faces are counted on the host (scalar sweeps of
-// larger levels do not ask).
+// Largest level whose active faces are counted on the host: at least the
+// largest that scalar_sweep_lanes_kernel takes, the only one to ask.
 constexpr int kActLevel = 16384;
 
-// Cells from which Pack goes through records.
+// Cells from which Pack goes through records.  They are faster at every size
+// (six variables, records / one pass, us, FP32 and FP64: 13.8K cells 12.4 / 24.7
+// and 12.5 / 18.3, 125K 24.6 / 49.3 and 21.7 / 34.8, 262K 38.7 / 67.6 and 49.4 /
+// 50.5, 885K 115 / 192 and 157 / 215); small systems, whose few us lie in the
+// launches of a step, do without the second copy of their state.
 constexpr long long kPackRecords = 131072;
 
 void pack_records_alloc(FlowSys s);
@@ -1228,9 +1232,8 @@ ucfd_status_t UCFDLUSGS_Pack(FlowSys s, UCFDInt eidx, UCFDReal turb_factor, UCFD
         if constexpr (std::is_same<S, float>::value) w.ulo.ensure((size_t)s->nvars * s->N);
         // one element of all cells: through records (several elements pack one
         // after the other into the same arrays, each with its own scattered
-        // pass).  Below kPackRecords cells, where no records are allocated, the
-        // scattered writes stay in L2 and one pass is faster.
-        // (Not into a graph, whose every launch would write the same stamp.)
+        // pass).  (Not into a graph, whose every launch would write the same
+        // stamp.)
         S *rec = w.rec.p;
         if (rec && e.neles == s->N && capture_id(s) == 0) {
             if (++s->pack_stamp <= 0) s->pack_stamp = 1;

@@ -375,7 +375,9 @@ __device__ __forceinline__ void split_add(const SweepSplit<S> &sp, int side, con
 
 // The other side's sum to start from: stored by the previous sweep in
 // partial mode (issued early, with the cell's other inputs), zero in full
-// mode.  In a dependent launch only after griddepcontrol.wait.
+// mode.  A level's part was last written by the previous sweep, which is
+// complete: the first launch of a sweep carries no dependent-launch attribute,
+// so the kept sums (and terms) may be read before griddepcontrol.wait too.
 template <typename S, int B>
 __device__ __forceinline__ void split_start(const SweepSplit<S> &sp, long long N, int var0, long long k, S *ta,
                                             S *to) {

@@ -135,7 +135,7 @@ __device__ __forceinline__ void ell_row_products(long long k, int bn, int P, con
 // 3 y = alpha A x, 0 the general form; 1 and 2 give the values of the general
 // form with alpha = 1, beta = 0 and alpha = -1, beta = 1 without its products
 // and, in FP64, without a comparison per row on the FP64 pipe.
-// VEC: x and y 16-byte aligned.
+// VEC: x is 16-byte aligned.
 template <typename Tv, typename Ta, int B, int PW, bool VEC>
 __global__ void __launch_bounds__(256) bsr_spmv_kernel(int bn, int P, const int *col, const Tv *val,
                                                        double alpha, const double *x, double beta,
@@ -158,9 +158,10 @@ __global__ void __launch_bounds__(256) bsr_spmv_kernel(int bn, int P, const int 
 
 // Values of a CSR-of-blocks array (row-major B x B blocks in slot order)
 // into the ELL-of-blocks layout: ELL entry (p, k) takes the block at slot
-// src[p*bn + k] (src < 0: padding, not written and never read), into out64 and / or out32 (rounded
-// to FP32) -- one pass for both, since reading the values is half of its
-// traffic.  A warp takes 32 consecutive rows of one p: it reads the blocks
+// src[p*bn + k] (src < 0: padding, not written; no product uses it, though a
+// later FP32 copy of the whole array converts what is there), into out64 and /
+// or out32 (rounded to FP32) -- one pass for both, since reading the values is
+// half of its traffic.  A warp takes 32 consecutive rows of one p: it reads the blocks
 // one after the other, its lanes along a block (whole sectors instead of one
 // 8-byte word of every row's block per load), into shared memory, then each
 // lane writes its row's values, coalesced over the rows.  Bound by HBM: 5.3M

@@ -148,8 +148,13 @@ static void sweep_both_go(const ::ucfd::ScalarSweepArgs<T> &a, int block, cudaSt
 // per cell and win while the sub-partitions (608) have few warps each.
 // Measured: natural-order FP64 step of 41x36x33 cells (108 levels of at most
 // 1100 cells, three active faces) 4.04 ms with one thread per cell in
-// blocks of 32, 0.91 ms with lanes chained by dependent launches.
-constexpr int kLanesCells4 = 12288, kLanesCells8 = 6144;
+// blocks of 32, 0.91 ms with lanes chained by dependent launches.  A lower +
+// upper pair of two colours, lanes / one thread per cell, exact mode:
+//   quadrilaterals (4): 4608 cells a colour 26.7 / 45.1 us, 8192 41.0 / 45.1,
+//     10368 55.3 / 47.1, 12800 59.5 / 45.2;
+//   hexahedra (8): 4000 47.1 / 69.6 us, 6083 67.9 / 71.7, 6912 77.8 / 69.7.
+// (FMA mode: 8192 36.9 / 43.0, 10368 49.0 / 44.6; 6083 61.4 / 63.6, 6912 67.6 / 63.5.)
+constexpr int kLanesCells4 = 8192, kLanesCells8 = 6144;
 
 template <int NV, int NFV, int NDIMS, int SYS>
 static void sweep_lanes_go(const ::ucfd::ScalarSweepArgs<double> &a, int gf, cudaStream_t s) {
@@ -172,7 +177,14 @@ static void sweep_lanes_go(const ::ucfd::ScalarSweepArgs<double> &a, int gf, cud
 // of a block's cells, whatever the launch variant's register cap.  Up to
 // kPackedMin cells one thread per cell has a sub-partition's FP64 pipe nearly
 // to itself, and the lists' barriers cost more than idle lanes (32^3 cells
-// in two colours of 16384: 191 us a step against 197).
+// in two colours of 16384: 191 us a step against 197).  What the lists gain
+// are the idle lanes of uneven cells.  Lower + upper pair of the greedy
+// colours of permuted hexahedra, exact mode, with the line at 8192 / 16384 /
+// 32768 / no lists: 40^3 cells (colours up to 20105) 223 / 225 / 250 / 250 us,
+// 48^3 (34692) 283 / 287 / 303 / 328, 56^3 (55242) 387 / 387 / 399 / 463, 64^3
+// (81893) 609 / 608 / 607 / 721.  Where every cell of a level has the same
+// faces (a checkerboard) there is nothing to gain and up to 2 % to lose:
+// colours of 19652 cells 104 us with lists, 103 without; 108000 395 and 385.
 constexpr int kPackedMin = 16384;
 
 template <int NV, int NFV, int NDIMS, int SYS>
@@ -523,6 +535,11 @@ static void sweep_small_go(cudaStream_t s, int t0, int t1, long long N, int var0
 // FP64 levels of at most this many cells take the kernel with B lanes per
 // cell: a warp then holds 32 / B cells and costs about 60 FP64 instructions
 // (fast build 32), against 270-420 (90) for 32 cells with one thread each.
+// A lower + upper pair of two colours of hexahedra, 5x5, lanes / one thread
+// per cell: 4000 cells a colour 23.6 / 56.9 us exact, 10.8 / 23.0 FMA; 7812
+// 48.0 / 84.5, 15.9 / 29.3; 16384 87.6 / 101, 29.0 / 34.3; 23328 116 / 105,
+// 32.9 / 37.8.  For these blocks the line could be at 16384; it is at half of
+// that for the narrower ones, with fewer lanes per cell, not measured.
 constexpr int kRowsCells = 8192;
 
 template <int B, int PW>
