@@ -577,12 +577,11 @@ bool still_holds(FlowSys s, unsigned long long then, unsigned long long now, boo
 // rhs when Pack or Prepare changed it, or a graph may have; the exact mode
 // sweeps rhs itself.
 template <typename S, bool EX>
-const S *sweep_rhs(FlowSys s, bool turb) {
+const S *sweep_rhs(FlowSys s, bool turb, unsigned long long now) {
     Work<S> &w = work<S>(s);
     if constexpr (EX) return w.rhs.p;
     const int B = turb ? s->ntvars : s->nfvars;
     const int var0 = turb ? s->nfvars : 0;
-    const unsigned long long now = block_capture_id(s);
     if (!s->c_valid[turb ? 1 : 0] || !still_holds(s, s->c_capture[turb ? 1 : 0], now, s->captured_inputs)) {
         w.crhs.ensure((size_t)s->nvars * s->N);
         kfast::fs_blusgs_rhs_solve<S>(B, s->N, var0, blu_LU<S>(s, turb), w.rhs.p, w.crhs.p, s->stream());
@@ -594,7 +593,7 @@ const S *sweep_rhs(FlowSys s, bool turb) {
 }
 
 template <typename S, bool EX>
-void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
+void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du, unsigned long long now) {
     Work<S> &w = work<S>(s);
     const int B = turb ? s->ntvars : s->nfvars;
     const int var0 = turb ? s->nfvars : 0;
@@ -605,7 +604,6 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
     // sweep in full mode)
     SweepSplit<S> sp;
     SplitState &ss = s->split[turb ? 1 : 0];
-    const unsigned long long now = block_capture_id(s);
     if constexpr (EX) {
         // nullptr (no room, or no sweep would read them): the terms are not kept
         sp.part = !s->has_self && still_holds(s, now, now, s->captured) ? w.spart.p : nullptr;
@@ -614,6 +612,7 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
         sp.part = w.spart.ensure((size_t)s->nvars * s->N);
     }
     sp.upper = upper ? 1 : 0;
+    sp.keep = sp.part ? sp.upper : -2;
     sp.nvars = s->nvars;
     sp.full = (!s->has_self && ss.du == du && ss.dir == (upper ? 0 : 1) && ss.ver == s->jver[turb ? 1 : 0] &&
                still_holds(s, ss.capture, now, s->captured)) ? 0 : 1;
@@ -646,13 +645,13 @@ void blusgs_sweep_into(FlowSys s, bool turb, bool upper, const S *rhs, S *du) {
 // du of the fast block sweeps was set to zero: both sides' sums are zero,
 // so the next lower sweep can start from stored (zero) sums.
 template <typename S>
-void split_zero(FlowSys s, bool turb, const S *du, cudaStream_t st) {
+void split_zero(FlowSys s, bool turb, const S *du, cudaStream_t st, unsigned long long now) {
     Work<S> &w = work<S>(s);
     const int B = turb ? s->ntvars : s->nfvars;
     const int var0 = turb ? s->nfvars : 0;
     w.spart.ensure((size_t)s->nvars * s->N);
     UCFD_CUDA(cudaMemsetAsync(w.spart.p + (size_t)var0 * s->N, 0, (size_t)B * s->N * sizeof(S), st));
-    s->split[turb ? 1 : 0] = SplitState{du, 1, s->jver[turb ? 1 : 0], nullptr, 0, block_capture_id(s)};
+    s->split[turb ? 1 : 0] = SplitState{du, 1, s->jver[turb ? 1 : 0], nullptr, 0, now};
 }
 
 void split_forget(FlowSys s) { s->split[0] = s->split[1] = SplitState{}; }
@@ -660,7 +659,8 @@ void split_forget(FlowSys s) { s->split[0] = s->split[1] = SplitState{}; }
 // Sweeps that one call makes one after the other: no graph runs in between.
 struct InCall {
     FlowSys s;
-    explicit InCall(FlowSys h) : s(h) {
+    const unsigned long long now;
+    explicit InCall(FlowSys h) : s(h), now(block_capture_id(h)) {
         if (s->captured) split_forget(s);
         if (s->captured_inputs) s->c_valid[0] = s->c_valid[1] = false;
         s->in_call = true;
@@ -1084,8 +1084,8 @@ ucfd_status_t UCFDFlowSysAutotune(FlowSys s, int reps, UCFDLaunchConfig *best) {
             InCall one(s);
             auto pair_ms = [&] {
                 return time_ms(st, reps, [&] {
-                    blusgs_sweep_into<S, EX>(s, false, false, w.rhs.p, scratch.p);
-                    blusgs_sweep_into<S, EX>(s, false, true, w.rhs.p, scratch.p);
+                    blusgs_sweep_into<S, EX>(s, false, false, w.rhs.p, scratch.p, one.now);
+                    blusgs_sweep_into<S, EX>(s, false, true, w.rhs.p, scratch.p, one.now);
                 });
             };
             // the unrolled kernels exist for ELL widths 6 and 4 only
@@ -1517,13 +1517,14 @@ static ucfd_status_t blusgs_sweep_api(FlowSys s, bool turb, bool upper) {
     need_mode(s, MODE_BLUSGS);
     build_topology(s);
     if (turb) UCFD_REQUIRE(s->ntvars > 0, "RANS sweep needs turbulence variables");
+    const unsigned long long now = block_capture_id(s);
     dispatch(s, [&]<typename S, bool EX>() {
         Work<S> &w = work<S>(s);
         UCFD_REQUIRE(w.rhs.p, "sweep before Pack");
         UCFD_REQUIRE(blu_LU<S>(s, turb), "sweep before Prepare");
-        blusgs_sweep_into<S, EX>(s, turb, upper, sweep_rhs<S, EX>(s, turb), w.bdu.p);
+        blusgs_sweep_into<S, EX>(s, turb, upper, sweep_rhs<S, EX>(s, turb, now), w.bdu.p, now);
     });
-    if (capture_id(s) == 0) {
+    if (now == 0) {
         s->du64_valid = false;
         s->x_zero = false;
     } else if (s->prec == UCFD_PREC_FP32) {
@@ -1545,6 +1546,7 @@ ucfd_status_t UCFDBLUSGS_Reset(FlowSys s) {
     build_topology(s);
     cudaStream_t st = s->stream();
     const size_t n = (size_t)s->nvars * s->N;
+    const unsigned long long now = block_capture_id(s);
     dispatch(s, [&]<typename S, bool EX>() {
         blusgs_alloc<S>(s);
         Work<S> &w = work<S>(s);
@@ -1552,13 +1554,13 @@ ucfd_status_t UCFDBLUSGS_Reset(FlowSys s) {
         w.dup.zero(n, st);
         if (std::is_same<S, float>::value) s->x64.zero(n, st);
         if constexpr (!EX) {
-            split_zero<S>(s, false, w.bdu.p, st);
-            if (s->ntvars > 0) split_zero<S>(s, true, w.bdu.p, st);
+            split_zero<S>(s, false, w.bdu.p, st, now);
+            if (s->ntvars > 0) split_zero<S>(s, true, w.bdu.p, st, now);
         } else {
             split_forget(s);  // the next sweep forms every term of the zero increments itself
         }
     });
-    if (block_capture_id(s) == 0) {  // (captured: du and x64 are both zero when it has run)
+    if (now == 0) {  // (captured: du and x64 are both zero when it has run)
         s->du64_valid = false;
         s->x_zero = true;
     }
@@ -1660,11 +1662,11 @@ ucfd_status_t UCFDBLUSGS_Solve(FlowSys s, UCFDReal rtol, UCFDInt max_sweeps, UCF
             kfast::fs_blusgs_rhs_solve<float>(s->nfvars, s->N, 0, w.LU.p, w.r.p, w.r.p, st);
             ++s->rver;
             w.delta.zero(n, st);
-            split_zero<float>(s, false, w.delta.p, st);
+            split_zero<float>(s, false, w.delta.p, st, one.now);
             const int m = std::min(inner_sweeps, max_sweeps - pairs);
             for (int q = 0; q < m; ++q) {
-                blusgs_sweep_into<float, false>(s, false, false, w.r.p, w.delta.p);
-                blusgs_sweep_into<float, false>(s, false, true, w.r.p, w.delta.p);
+                blusgs_sweep_into<float, false>(s, false, false, w.r.p, w.delta.p, one.now);
+                blusgs_sweep_into<float, false>(s, false, true, w.r.p, w.delta.p, one.now);
             }
             pairs += m;
             kfast::axpy_into<float>((long long)n, w.delta.p, s->x64.p, st);
@@ -1686,12 +1688,12 @@ ucfd_status_t UCFDBLUSGS_Solve(FlowSys s, UCFDReal rtol, UCFDInt max_sweeps, UCF
             const int m = std::min(inner_sweeps, max_sweeps - pairs);
             for (int q = 0; q < m; ++q) {
                 if (ex) {
-                    blusgs_sweep_into<double, true>(s, false, false, w.rhs.p, w.bdu.p);
-                    blusgs_sweep_into<double, true>(s, false, true, w.rhs.p, w.bdu.p);
+                    blusgs_sweep_into<double, true>(s, false, false, w.rhs.p, w.bdu.p, one.now);
+                    blusgs_sweep_into<double, true>(s, false, true, w.rhs.p, w.bdu.p, one.now);
                 } else {
-                    const double *c = sweep_rhs<double, false>(s, false);
-                    blusgs_sweep_into<double, false>(s, false, false, c, w.bdu.p);
-                    blusgs_sweep_into<double, false>(s, false, true, c, w.bdu.p);
+                    const double *c = sweep_rhs<double, false>(s, false, one.now);
+                    blusgs_sweep_into<double, false>(s, false, false, c, w.bdu.p, one.now);
+                    blusgs_sweep_into<double, false>(s, false, true, c, w.bdu.p, one.now);
                 }
             }
             pairs += m;

@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(256) fs_blusgs_sweep_kernel(int t0, int t1, lo
             for (int c = 1; c < B; ++c) val += __ldcs(Jp + ((r * B + c) << 5)) * x[c];
             val *= fv;
             b[r] -= val;
-            if (sd == sp.upper && sp.part) term[r * N] = val;
+            if (sd == sp.keep) term[r * N] = val;
         }
     };
     if constexpr (PW > 0) {
@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(32) fs_blusgs_sweep_rows_kernel(int t0, int t1
         const int sd = nb[p] >= 0 ? split_side(nb[p], t0, t1) : -1;
         const bool u = sd >= 0 && split_uses(sp, sd);
         use |= u ? 1u << p : 0u;
-        own |= sd == sp.upper ? 1u << p : 0u;
+        own |= sd == (kFold ? sp.upper : sp.keep) ? 1u << p : 0u;
         if (u) {
 #pragma unroll
             for (int q = 0; q < B; ++q) jv[p][q] = __ldcs(Jr + ((p * B2 + q) << 5));
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(32) fs_blusgs_sweep_rows_kernel(int t0, int t1
             for (int q = 1; q < B; ++q) val += jv[p][q] * x[p][q];
             val *= f[p];
             b -= val;
-            if (valid && sp.part && (own >> p) & 1u) sp.part[((long long)p * sp.nvars + var0 + r) * N + k] = val;
+            if (valid && (own >> p) & 1u) sp.part[((long long)p * sp.nvars + var0 + r) * N + k] = val;
         } else if (nb[p] >= 0) {
             b -= kept[p];
         }
