@@ -25,9 +25,10 @@ __device__ __forceinline__ T ld_once(const T *p) {
 // costs the L1 one pass per lane whatever its width: a row is read with the
 // fewest loads its alignment allows.
 //   FP64, B = XS = 5, VEC (base 16-byte aligned): two 16-byte loads and one
-//     8-byte load, the odd entry first in odd rows (the FP32 matvec, 5.3M
-//     rows: 711 -> 586 us with the conversions below; the FP64 kernels, bound
-//     by the FP64 pipe, gain nothing from it and do not use it);
+//     8-byte load, the odd entry first in odd rows (the FP32 matvec in the
+//     mixed solve of 5.3M rows: 0.70 -> 0.66 ms a launch with the conversions
+//     on the integer pipe; the FP64 kernels, bound by the FP64 pipe, gain
+//     nothing from it and do not use it);
 //   FP32, XS = 8: one 16-byte load and one per entry above 4;
 //   else one load per entry.
 template <typename Tx, int B, int XS, bool VEC>
