@@ -160,7 +160,10 @@ UCFD_EXTERN ucfd_status_t UCFDFlowSysSetLaunchConfig(FlowSys sys, const UCFDLaun
  * calls of a handle have been captured, its uncaptured sweeps form every face
  * (for as long as the handle lives; Solve keeps them within its own call).
  * UCFD_PREC_FP32: an Update captured without a sweep before it in the same
- * graph adds the FP32 increments, also after a Solve. */
+ * graph adds the FP32 increments, also after a Solve; NSRANS sweeps read the
+ * two systems' radii packed only under the same rule.  A LU-SGS Update does
+ * what the Pack or Run called or captured before it asks for: capture it with
+ * its Pack. */
 UCFD_EXTERN ucfd_status_t UCFDFlowSysSetStream(FlowSys sys, void *cuda_stream, int async);
 
 /* Scalar LU-SGS pseudo-time loop on device-resident state: niter times

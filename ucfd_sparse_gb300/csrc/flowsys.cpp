@@ -118,6 +118,8 @@ struct _FlowSys {
     bool has_self = false;         // some CSR row lists itself
     std::vector<int> act[2];       // per level: most faces of a cell towards earlier / later levels (0: not known)
     bool lam2_ok = false;          // Work::lam2 packs the current NS and RANS spectral radii (FP32)
+    unsigned long long lam2_capture = 0;  // the capture that packed it (as SplitState::capture)
+    bool lusgs_captured = false;   // a Prepare or sweep of the scalar path was captured (as captured)
     DevBuf<double> part, red, resid;
     PinnedBuf<double> h_red;
 
@@ -318,6 +320,24 @@ void need_mode(FlowSys s, int m) {
     if (s->mode != m)
         fail(UCFD_ERR_STATE, "FlowSys is not set up for %s (call UCFDFlowSysSet%s first)",
              m == MODE_LUSGS ? "LU-SGS" : "BLU-SGS", m == MODE_LUSGS ? "LUSGS" : "BLUSGS");
+}
+
+// The capture that the handle's stream is under: the call's work then runs
+// when (and as often as) the graph is launched, not now.  0: none.
+unsigned long long capture_id(FlowSys s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(s->stream(), &st, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return ~0ull;
+    }
+    return st == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
+// Whether what a call under capture `then` left on the device is still there
+// for a call under capture `now`; graphs: some may run in between.
+bool still_holds(FlowSys s, unsigned long long then, unsigned long long now, bool graphs) {
+    return then == now && (now != 0 || !graphs || s->in_call);
 }
 
 // ---- scalar LU-SGS --------------------------------------------------------
@@ -540,18 +560,6 @@ const S *blu_LU(FlowSys s, bool turb) {
     else return turb ? s->w32.tLU.p : s->w32.LU.p;
 }
 
-// The capture that the handle's stream is under: the call's work then runs
-// when (and as often as) the graph is launched, not now.  0: none.
-unsigned long long capture_id(FlowSys s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    unsigned long long id = 0;
-    if (cudaStreamGetCaptureInfo(s->stream(), &st, &id) != cudaSuccess) {
-        cudaGetLastError();
-        return ~0ull;
-    }
-    return st == cudaStreamCaptureStatusNone ? 0 : id;
-}
-
 // The same for a call of the block path, which notes that there is one.
 unsigned long long block_capture_id(FlowSys s) {
     const unsigned long long id = capture_id(s);
@@ -564,12 +572,6 @@ unsigned long long input_capture_id(FlowSys s) {
     const unsigned long long id = block_capture_id(s);
     s->captured_inputs = s->captured_inputs || id != 0;
     return id;
-}
-
-// Whether what a call under capture `then` left on the device is still there
-// for a call under capture `now`; graphs: some may run in between.
-bool still_holds(FlowSys s, unsigned long long then, unsigned long long now, bool graphs) {
-    return then == now && (now != 0 || !graphs || s->in_call);
 }
 
 // Right-hand side of the fast modes' block sweeps (their blocks are
@@ -790,6 +792,7 @@ void pack_both(FlowSys s, cudaStream_t st) {
         kfast::pack_lam2(nl, w.lamN.p, w.lamT.p, w.lam2.ensure((size_t)nl), st);
         pack_geo<S>(s, st);
         s->lam2_ok = true;
+        s->lam2_capture = 0;
     }
 }
 
@@ -1320,6 +1323,8 @@ static ucfd_status_t lusgs_prepare_api(FlowSys s, int sys, UCFDReal kappa) {
               w.diag.p, st);
         if (lam2) pack_geo<S>(s, st);
         s->lam2_ok = lam2 != nullptr;
+        s->lam2_capture = capture_id(s);
+        s->lusgs_captured = s->lusgs_captured || s->lam2_capture != 0;
     });
     finish(s, (lfN && !is_device_ptr(s->fspr)) || (lfT && !is_device_ptr(s->tfspr)));
     UCFD_API_END
@@ -1330,6 +1335,11 @@ static ucfd_status_t lusgs_sweep_api(FlowSys s, int sys, bool upper, UCFDReal ka
     need_mode(s, MODE_LUSGS);
     build_topology(s);
     if (sys != 0) UCFD_REQUIRE(s->ntvars > 0, "RANS sweep needs turbulence variables (nvars > nfvars)");
+    // the packed radii, where no graph can have run a Prepare since (the
+    // radii of each system by itself are those of whatever Prepare ran last)
+    const unsigned long long now = capture_id(s);
+    s->lusgs_captured = s->lusgs_captured || now != 0;
+    const bool packed = sys == 2 && still_holds(s, s->lam2_capture, now, s->lusgs_captured);
     dispatch(s, [&]<typename S, bool EX>() {
         Work<S> &w = work<S>(s);
         UCFD_REQUIRE(w.du.p, "sweep before Pack");
@@ -1341,7 +1351,7 @@ static ucfd_status_t lusgs_sweep_api(FlowSys s, int sys, bool upper, UCFDReal ka
             lusgs_sweep<S, EX>(s, 0, upper, kappa);
             lusgs_sweep<S, EX>(s, 1, upper, kappa);
         } else {
-            lusgs_sweep<S, EX>(s, sys, upper, kappa, false, sys == 2);
+            lusgs_sweep<S, EX>(s, sys, upper, kappa, false, packed);
         }
     });
     finish(s);
